@@ -141,13 +141,37 @@ __device__ __forceinline__ double block_min(double v, double* scratch) {
     return -block_max(-v, scratch);
 }
 
+// a / b correctly rounded, rb = RN(1 / b) (__drcp_rn), for dividing many
+// values by one divisor: Markstein's quotient refinement (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990: with rb correctly rounded and q
+// within an ulp of a / b, q + rb * (a - b q), the remainder exact by fma, is
+// RN(a / b)).  The first refinement brings a * rb within that ulp.  Outside
+// exponents +-400 of either operand (where an intermediate could leave the
+// normal range), and for a non-finite one, the division itself.  A zero keeps
+// its sign.  Why: a dependent chain of 40 cycles after the reciprocal (61);
+// __ddiv_rn takes 420 for a warp with one zero dividend (measured, B200).
+static __device__ __noinline__ double div_call(double a, double b) { return __ddiv_rn(a, b); }
+__device__ __forceinline__ double div_by(double a, double b, double rb) {
+    const double q0 = __dmul_rn(a, rb);
+    const double q1 = fma(fma(-b, q0, a), rb, q0);
+    const double q2 = fma(fma(-b, q1, a), rb, q1);
+    const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eb = ((unsigned)__double2hiint(b) >> 20) & 0x7ffu;
+    const bool in = eb - 623u <= 800u;
+    if (in && ea - 623u <= 800u) return q2;
+    if (in && a == 0.0) return q0;
+    return div_call(a, b);   // a call: the expansion stays out of unrolled loops
+}
+
 template <typename T> struct ValTraits;
 template <> struct ValTraits<double> {
     static __device__ __forceinline__ double load(const double* p) { return *p; }
+    static __device__ __forceinline__ double load_cg(const double* p) { return __ldcg(p); }
     static __device__ __forceinline__ double to(double v) { return v; }
 };
 template <> struct ValTraits<float> {
     static __device__ __forceinline__ double load(const float* p) { return (double)*p; }
+    static __device__ __forceinline__ double load_cg(const float* p) { return (double)__ldcg(p); }
     static __device__ __forceinline__ float to(double v) { return (float)v; }
 };
 

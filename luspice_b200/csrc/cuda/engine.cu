@@ -583,21 +583,23 @@ void make_dense_plan(const std::vector<PatternObj*>& pats, int threads, SmemPlan
     const size_t budget = 227 * 1024;
     plan.bytes = fixed;
     if (dmax == 0) return;
-    // Panel [D][nb + 1] (padded rows) + U tile [nb][128] + per-warp column
-    // maxima [nb][32] + 4 cycle counters: the widest panel (32, 16, 8) that
-    // fits.
-    auto dneed = [&](int nb) { return fixed + 8 * ((size_t)dmax * (nb + 1) + (size_t)nb * 128 + (size_t)nb * 32 + 4); };
-    int nb = 32;
-    while (nb > 8 && dneed(nb) > budget) nb /= 2;
-    plan.tnb = nb;
-    plan.bytes = dneed(nb);
-    // The transpose reuses the area: a padded 32 x 33 fp64 tile per warp.
-    const size_t tile_b = 32 * 33 * sizeof(double);
-    int ttw = (int)std::min<size_t>({(size_t)threads / 32, 16, (budget - fixed) / tile_b});
-    ttw = std::max(1, ttw);
-    plan.ttw = ttw;
-    plan.bytes = std::max(plan.bytes, fixed + ttw * tile_b);
+    // Block column [D][33], pivot rows [32][34], panel row groups in flight
+    // (1 KB each; three per updating warp where they fit), where the column
+    // maxima of the panel phase also live.
+    const int nup = threads / 32 - 1;
+    plan.drows = (dmax + 31) & ~31;
+    auto dneed = [&](int stg) {
+        return fixed + 8 * ((size_t)plan.drows * 33 + 32 * 34 + (size_t)nup * stg * 128);
+    };
+    plan.dstg = dneed(3) <= budget ? 3 : 1;
+    plan.bytes = dneed(plan.dstg);
 }
+
+// CTA size of the dense-block kernel when a lone CTA takes a system: a
+// thread per row of the block, up to 512, so that small blocks share an SM
+// (768 circuits with D up to 128, B200: four CTAs of 128 threads per SM
+// 0.27 ms; the block's chain, not its arithmetic, fills a CTA's time).
+static int dense_block_threads(int dmax) { return dmax <= 128 ? 128 : dmax <= 256 ? 256 : 512; }
 
 // Raise the dynamic shared-memory limit of one kernel (once per size; not a
 // stream operation, so it stays out of captured graphs after the first
@@ -1047,17 +1049,12 @@ int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& 
     a.dblock = 512;
     a.dgrid = 0;
     if (ntail > 0) {
-        make_dense_plan(pats, a.dblock, a.dplan);
-        int docc = 0;
-        rc = o.prec == LUSP_FP64 ? dense_prepare<double>(a.dplan.bytes, a.dblock, &docc)
-                                 : dense_prepare<float>(a.dplan.bytes, a.dblock, &docc);
-        if (rc != LUSP_OK) return rc;
-        if (docc < 1) { set_error("dense kernel does not fit one SM (smem %zu)", a.dplan.bytes); return LUSP_EARG; }
-        a.dgrid = std::min(ntail, docc * sm_count());
-        // Two CTAs per block (a 2-CTA cluster that splits the trailing
-        // updates) when every system with a block gets its pair of SMs.
+        // Two CTAs of 512 threads per block (a 2-CTA cluster whose CTAs take
+        // the block columns in turn) when every system with a block gets its
+        // pair of SMs.
         a.dcluster = 1;
-        if (a.dplan.tnb == 32 && 2 * ntail <= sm_count()) {
+        if (2 * ntail <= sm_count()) {
+            make_dense_plan(pats, a.dblock, a.dplan);
             int ncl = 0;
             rc = o.prec == LUSP_FP64 ? dense_cluster_count<double>(a.dplan.bytes, a.dblock, &ncl)
                                      : dense_cluster_count<float>(a.dplan.bytes, a.dblock, &ncl);
@@ -1066,6 +1063,17 @@ int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& 
                 a.dcluster = 2;
                 a.dgrid = 2 * ntail;
             }
+        }
+        if (a.dcluster == 1) {
+            int dmax = 0, docc = 0;
+            for (auto* p : pats) dmax = std::max(dmax, p->S.dtail);
+            a.dblock = dense_block_threads(dmax);
+            make_dense_plan(pats, a.dblock, a.dplan);
+            rc = o.prec == LUSP_FP64 ? dense_prepare<double>(a.dplan.bytes, a.dblock, &docc)
+                                     : dense_prepare<float>(a.dplan.bytes, a.dblock, &docc);
+            if (rc != LUSP_OK) return rc;
+            if (docc < 1) { set_error("dense kernel does not fit one SM (smem %zu)", a.dplan.bytes); return LUSP_EARG; }
+            a.dgrid = std::min(ntail, docc * sm_count());
         }
     }
     return LUSP_OK;

@@ -45,8 +45,8 @@ struct PatternDev {
                                   // strict-L length} of the dependency column
     const unsigned short* rel;    // relative update slots (null: search rows)
     const long long* rel_ptr;     // [n+1] column k's list in rel
-    // Dense trailing block: rows/columns [k0, n), dtail = n - k0 (0: none),
-    // stored row-major with leading dimension tail_ld.
+    // Dense trailing block: rows/columns [k0, n), dtail = n - k0 (0: none);
+    // tail_ld: dtail rounded up to 32.
     int k0, dtail, tail_ld;
     // Pattern of the dense trailing block, one bit per entry (row r, column c
     // of the block: bit c & 31 of word r * (tail_ld / 32) + c / 32).  The
@@ -114,7 +114,7 @@ struct SysDev {
     void* tail;              // [dtail * tail_ld] dense L\U of the trailing
                              // block (VT, column-major: (i, c) at c * ld + i),
                              // unit L below the diagonal
-    double* tailw;           // [dtail * tail_ld] fp64 trailing block (row-major)
+    double* tailw;           // [dtail * tail_ld] fp64 trailing block (tail_index)
                              // between the refactor and dense kernels
     void* tinv;              // [ceil(dtail/32) * 2048] inverses of the dense
                              // block's 32 x 32 diagonal blocks (VT): per block
@@ -135,6 +135,13 @@ struct SolveParams {
 };
 
 constexpr int kMaxKrylov = 64;
+
+// Entry (r, c) of a dense trailing block of D rows in the fp64 work copy:
+// block columns of 32, each contiguous, row after row (a block column and
+// the rows of a panel are then single runs of memory).
+__host__ __device__ inline size_t tail_index(int D, int r, int c) {
+    return ((size_t)(c >> 5) * D + r) * 32 + (c & 31);
+}
 
 // Sizes that fix one system's private device area.
 struct SysSizes {
@@ -229,8 +236,8 @@ struct SmemPlan {
     int nwords;              // ready-bit words (>= ceil(n_max/32))
     int wcap;                // per-warp refactor work slots
     int scap;                // per-warp staged L entries (refactor gathers)
-    int tnb;                 // panel width of the dense trailing block
-    int ttw;                 // warps transposing the dense block (32x33 fp64 tile each)
+    int drows;               // dense trailing block: rows of a block column
+    int dstg;                // ... and panel row groups in flight per warp (1 or 3)
     int sc_ent, sc_rows;     // sweep stage capacity (entries, rows; 0: no stages)
     int ycap;                // doubles for a shared-memory solve vector
     int dcap;                // ints for shared-memory sweep descriptors

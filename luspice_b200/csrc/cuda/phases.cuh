@@ -55,6 +55,10 @@ __device__ __forceinline__ void cp_async_8(void* sdst, const void* gsrc) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
+__device__ __forceinline__ void cp_async_16(void* sdst, const void* gsrc) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
+}
 __device__ __forceinline__ void cp_async_val(float* sdst, const float* gsrc) { cp_async_4(sdst, gsrc); }
 __device__ __forceinline__ void cp_async_val(double* sdst, const double* gsrc) { cp_async_8(sdst, gsrc); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
@@ -142,455 +146,488 @@ __device__ void cta_store_pivot_stats(SysStats* st, Smem& sm, double minpiv, dou
 }
 
 // ---------------------------------------------------------------------------
-// Dense trailing block of the refactorization (rows and columns [k0, n)),
-// in place in W (fp64, row-major, leading dimension ld).  On entry W holds
-// the block after the updates from the columns before k0; on exit its strict
-// lower part holds the stored (VT-rounded) multipliers and its upper part
-// the fp64 U values.  Right-looking with panels of nb columns (the panel in
-// shared memory): entry (i, c) still receives its updates in ascending order
-// of the pivot column, each a separately rounded multiply and subtract with
-// the stored multiplier and the fp64 U value, so the factor equals the
-// column engine's bit for bit.  Pivot statistics as in the column engine.
+// Dense trailing block of the refactorization (rows and columns [k0, n)).
+// On entry W (fp64, block columns of 32: entry (r, c) at tail_index) holds
+// the block after the updates from the columns before k0, in the entries of
+// its pattern; the rest of W is undefined and read as 0.
+//
+// Left-looking by block columns of 32.  A CTA holds one block column in
+// shared memory ([D][33] fp64), applies the finished panels before it, and
+// factors it as the next panel.  An entry receives its updates in ascending
+// order of the pivot column, each a separately rounded multiply and subtract
+// with the stored (VT-rounded) multiplier and the fp64 U value, so the
+// factor equals the column engine's bit for bit.  Pivot statistics as in the
+// column engine.
+//
+// What bounds it: the chain panel -> update of the next block column ->
+// next panel.  A panel column costs one division, one barrier and the
+// pivot row's broadcast because a thread keeps its row of the panel in
+// registers (measured below); the updates run at the fp64 pipe's rate
+// because a lane keeps its column of the panel's U block in registers and
+// the multipliers are broadcast from shared memory (one 16-byte load per two
+// multiply-subtract pairs of a warp).  Warps other than the last stream
+// their own rows of the panel (four rows of 256 bytes per copy group) with
+// no CTA barrier; the last warp solves the next panel's 32 x 32 unit-lower
+// block for U meanwhile.  CL: the two CTAs of a cluster take the block
+// columns in turn; a finished panel is published through W (L2) and a
+// counter in both CTAs' shared memory.
+// B200, event times per launch: 50 systems with D = 320 (n = 4050 grid)
+// 0.652 -> 0.438 ms, one system with D = 96 (n = 113 circuit) 155 -> 94 us,
+// 768 systems with D up to 128 on lone CTAs 0.70 -> 0.27 ms, against a
+// right-looking version with the panel in shared memory (a lane per row,
+// 1.4-1.7 k cycles a column) and the trailing block in global memory.  The
+// floor is the fp64 pipe: D^3 / 3 pairs at 32 per cycle and SM, 90 us for
+// D = 320 on two SMs.
 // ---------------------------------------------------------------------------
-// Entry (r, c) of the dense trailing block W, or 0 when it is outside the
-// block's pattern (first panel step only: the refactor wrote the pattern
-// entries alone, the rest of W holds whatever an earlier launch left).
-// Split thread-block cluster barrier (every thread of both CTAs arrives,
-// then waits; release / acquire at cluster scope).
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void named_sync(int id, int threads) {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int threads) {
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+// Named barriers of the dense kernel: U block of a panel ready, rows of the
+// next U block updated, and one for each four pivot rows of a panel.
+constexpr int kBarU = 1, kBarRows = 2, kBarPivots = 3;
+// Control word of Smem::ctl: panels finished (both CTAs of a cluster).
+constexpr int kCtlPanels = 8;
 
-template <bool CG = false>
-__device__ __forceinline__ double tail_entry(const double* W, int ld, const unsigned* mask, int r, int c,
-                                             bool masked) {
-    if (masked && !((__ldg(mask + (size_t)r * (ld >> 5) + (c >> 5)) >> (c & 31)) & 1u)) return 0.0;
-    return CG ? __ldcg(W + (size_t)r * ld + c) : W[(size_t)r * ld + c];
+// Bounded wait until the published panels reach `want` (every lane of a warp
+// calls; the acquire orders the panel's reads after it).
+__device__ __forceinline__ bool dense_wait_panel(int* ctl, int want, bool cluster) {
+    const volatile int* done = ctl + kCtlPanels;
+    const volatile int* ab = ctl + 3;
+    bool ok = true;
+    for (long long it = 0; *done < want; it++) {
+        if (*ab || it > kSpinLimit) {
+            atomicExch(ctl + 3, 1);
+            ok = false;
+            break;
+        }
+        __nanosleep(20);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    share_fence(cluster ? 2u : 1u);
+    return ok;
 }
 
-// CL: the block is shared by the two CTAs of a thread-block cluster.  Rank
-// 0 factors each panel alone, one step ahead (look-ahead); rank 1 copies it
-// from rank 0's shared memory.  In each step rank 0 takes the U rows and the
-// trailing update of the next panel's columns, rank 1 those of all other
-// columns, so each column of W is written by one CTA between two cluster
-// barriers.  W is then read through L2 (ld.cg), where the other CTA's writes
-// are, never from a stale L1 line.
-template <typename VT, bool CL = false>
-__device__ void dense_tail_factor(const PatternDev& P, double* W, Smem& sm, const SmemPlan& plan,
-                                  const SolveParams& prm, double& minpiv, double& minratio, int& bad,
-                                  SysStats* st) {
-    namespace cgr = cooperative_groups;
-    const int crank = CL ? (int)cgr::this_cluster().block_rank() : 0;
-    const bool lead = crank == 0;
-    const int D = P.dtail, ld = P.tail_ld, k0 = P.k0, nb = plan.tnb;
-    const int ps = nb + 1;   // panel row stride: odd, so a lane per row hits distinct banks
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
-    double* pan = (double*)sm.uni;                                           // [D][ps]
-    double* ut = pan + (size_t)D * ps;                                       // [nb][128]
-    // Per column of the panel, each warp's maximum |L| before scaling (the
-    // pivot statistics' denominator): a slot per warp, reduced after the
-    // panel, so the panel's column chain carries no atomics.
-    double* wmax = ut + (size_t)nb * 128;                                    // [nb][32]
-    long long* ctr = (long long*)(wmax + (size_t)nb * 32);   // [4] stage cycles (thread 0)
-    if (tid == 0) {
-        ctr[0] = ctr[1] = ctr[2] = 0;
-        ctr[3] = clock64();
+// Four rows (1 KB, contiguous) of a finished panel into shared memory, two
+// 16-byte pieces per lane that bypass L1 (another SM may have written them).
+__device__ __forceinline__ void dense_copy_rows(double* dst, const double* src, int rows) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int piece = lane + 32 * q;   // 16 pieces per row
+        if ((piece >> 4) < rows) cp_async_16(dst + 2 * piece, src + 2 * piece);
     }
-    const unsigned* mask = P.tail_mask;
-    auto wld = [W](size_t i) { return CL ? __ldcg(W + i) : W[i]; };
-    const int warp = tid >> 5, nw = nt >> 5;
-    // Panel jb: loaded into shared memory, factored, its pivot statistics
-    // taken and written back to W (rank 0 alone in a cluster).
-    auto panel = [&](int jb) {
-        const int w = min(nb, D - jb), R = D - jb;
-        const bool first = jb == 0;
-        for (int t = tid; t < R * nb; t += nt) {
-            const int r = t / nb, c = t - r * nb;
-            pan[r * ps + c] = c < w ? tail_entry<CL>(W, ld, mask, jb + r, jb + c, first) : 0.0;
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// The phases below keep a row or a column of 32 fp64 values in registers;
+// each is a call, so its registers are its own.  The substitutions are rolled
+// loops over groups of four pivots whose update writes entry q to register
+// q - 4: 4.8 k cycles for 32 columns (B200) with an eighth of the unrolled
+// instructions; over single pivots 7.3 k (the loop's branches and the
+// shared-memory latency are paid 32 times instead of 8).
+//
+// Forward substitution with the lower triangle at lk (row r at lk + pitch r),
+// one column per lane in u.  EXACT: unit diagonal, separately rounded
+// multiply and subtract (U rows of a panel); the solution of row r goes to
+// out[33 r].  Else fma and a division by the diagonal (its reciprocal at
+// lk + pitch r + 32): inverses, stored as VT to out[r * step].
+template <bool EXACT, typename OT>
+__device__ __forceinline__ void dense_substitute(const double* lk, int pitch, double (&u)[32], OT* out, int step) {
+    auto sub = [](double a, double l, double x) { return EXACT ? __dsub_rn(a, __dmul_rn(l, x)) : fma(-l, x, a); };
+#pragma unroll 1
+    for (int c = 0; c < 32; c += 4) {
+        const double* lc = lk + (size_t)c * pitch + c;   // L[c + i][c + k] at lc + pitch i + k
+        auto fin = [&](int i) {
+            if (!EXACT) u[i] = div_by(u[i], lc[(size_t)i * pitch + i], lk[(size_t)(c + i) * pitch + 32]);
+        };
+        fin(0);
+#pragma unroll
+        for (int i = 1; i < 4; i++) {
+#pragma unroll
+            for (int k = 0; k < i; k++) u[i] = sub(u[i], lc[(size_t)i * pitch + k], u[k]);
+            fin(i);
         }
-        __syncthreads();
-        // Panel: unblocked elimination, a lane per row and a warp per 32
-        // rows, so a row's multiplier and its update stay inside one warp:
-        // one CTA barrier per column (the pivot row must be final for all).
-        for (int c = 0; c < w; c++) {
-            const double piv = pan[c * ps + c];
-            const double* urow = pan + (size_t)c * ps;
-            double lm = 0.0;
-            for (int r0 = c + 1 + warp * 32; r0 < R; r0 += nw * 32) {
-                const int r = r0 + lane;
-                if (r < R) {
-                    double* row = pan + (size_t)r * ps;
-                    const double v = row[c];
-                    lm = fmax(lm, fabs(v));
-                    const double l = (double)ValTraits<VT>::to(__ddiv_rn(v, piv));
-                    row[c] = l;
-                    // Eight entries and their pivot-row values are loaded
-                    // before any is stored (the stores could alias the loads).
-                    for (int j0 = c + 1; j0 < w; j0 += 8) {
-                        double a[8], u[8];
+        const double u0 = u[0], u1 = u[1], u2 = u[2], u3 = u[3];
+        out[(c + 0) * step] = ValTraits<OT>::to(u0);
+        out[(c + 1) * step] = ValTraits<OT>::to(u1);
+        out[(c + 2) * step] = ValTraits<OT>::to(u2);
+        out[(c + 3) * step] = ValTraits<OT>::to(u3);
 #pragma unroll
-                        for (int q = 0; q < 8; q++) {
-                            a[q] = j0 + q < w ? row[j0 + q] : 0.0;
-                            u[q] = j0 + q < w ? urow[j0 + q] : 0.0;
-                        }
+        for (int m = 4; m < 32; m += 4) {
+            if (m < 32 - c) {
 #pragma unroll
-                        for (int q = 0; q < 8; q++)
-                            if (j0 + q < w) row[j0 + q] = __dsub_rn(a[q], __dmul_rn(l, u[q]));
+                for (int q = m; q < m + 4; q++) {
+                    const double2 a = *(const double2*)(lc + (size_t)q * pitch);
+                    const double2 b = *(const double2*)(lc + (size_t)q * pitch + 2);
+                    u[q - 4] = sub(sub(sub(sub(u[q], a.x, u0), a.y, u1), b.x, u2), b.y, u3);
+                }
+            }
+        }
+    }
+}
+
+// u := L^-1 u for the unit-lower 32 x 32 block at lk (row r at lk + 32 r),
+// one column per lane (u[r] at xk + 33 r).
+__device__ __noinline__ void dense_solve_unit(const double* lk, double* xk) {
+    double u[32];
+#pragma unroll
+    for (int r = 0; r < 32; r++) u[r] = xk[r * 33];
+    dense_substitute<true>(lk, 32, u, xk, 33);
+}
+
+// Inverse of the 32 x 32 lower triangle at lk (row r at lk + 34 r, reciprocal
+// diagonal at lk + 34 r + 32), a column per lane: element (r, lane) as VT at
+// out[r * step].
+template <typename VT>
+__device__ __noinline__ void dense_block_inverse(const double* lk, VT* out, int step) {
+    const int lane = threadIdx.x & 31;
+    double u[32];
+#pragma unroll
+    for (int r = 0; r < 32; r++) u[r] = r == lane ? 1.0 : 0.0;
+    dense_substitute<false>(lk, 34, u, out, step);
+}
+
+// Rows [rb, D) of the block column xs minus the panel rows src (row r at
+// src + 32 r) times the panel's U block (column of this lane at xk + 33 c),
+// four rows per group, groups warp, warp + nup, ...; my: this warp's stages.
+// told: barrier kBarRows needs no arrival after this warp's groups below 8.
+__device__ __noinline__ void dense_update_rows(double* xs, const double* xk, const double* src, double* my, int rb,
+                                               int D, int nup, int stg, int nt, bool told) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ng = (D - rb + 3) >> 2;
+    auto issue = [&](int g, int slot) {
+        if (g < ng) dense_copy_rows(my + slot * 128, src + (size_t)(rb + 4 * g) * 32, D - rb - 4 * g);
+        else asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    for (int t = 0; t < stg; t++) issue(warp + t * nup, t);
+    named_sync(kBarU, nt);
+    double u[32];
+#pragma unroll
+    for (int c = 0; c < 32; c++) u[c] = xk[c * 33];
+    int slot = 0;
+    for (int g = warp; g < ng; g += nup) {
+        if (!told && g >= 8) {
+            named_arrive(kBarRows, 32 * (min(8, nup) + 1));
+            told = true;
+        }
+        if (stg >= 3) asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncwarp();
+        const double* l = my + slot * 128;
+        const int row = rb + 4 * g;
+        double a[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) a[q] = xs[(size_t)min(row + q, D - 1) * 33 + lane];
+#pragma unroll
+        for (int c = 0; c < 32; c += 2) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const double2 lv = *(const double2*)(l + q * 32 + c);
+                a[q] = __dsub_rn(a[q], __dmul_rn(lv.x, u[c]));
+                a[q] = __dsub_rn(a[q], __dmul_rn(lv.y, u[c + 1]));
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (row + q < D) xs[(size_t)(row + q) * 33 + lane] = a[q];
+        __syncwarp();
+        issue(g + stg * nup, slot);
+        slot = slot + 1 < stg ? slot + 1 : 0;
+    }
+    if (!told) named_arrive(kBarRows, 32 * (min(8, nup) + 1));
+    cp_async_wait_all();
+    __syncwarp();
+}
+
+// A panel of R rows (row r at xj + 33 r) and w columns.  Warp 0 factors the
+// 32 pivot rows alone (a row per lane in registers, the pivot row exchanged
+// through shared memory); the other warps (a row per lane, rows past the
+// CTA's threads in later passes) follow four columns behind it, held only by
+// one named barrier per four columns.  Their loop writes entry q to register
+// q - 4, so it is rolled and the current columns are registers 0..3.  Bound by
+// warp 0's chain (exchange, reciprocal 61, quotient 50, update 16 cycles a
+// column, and its own update's issue): 320 rows and 32 columns 24 k cycles
+// (B200); all warps in step, a barrier per column, 39 k; groups of four
+// pivots eliminated redundantly by every lane 34 k (two dependent divisions
+// per column instead of one).
+// ud: the pivot rows, entry (r, 4 (r / 4) + q) at ud + 34 r + q, the pivot's
+// reciprocal at ud + 34 r + 32.  vmax[c]: bits of the largest entry of column
+// c below the pivot before scaling, over the entries whose multiplier is at
+// least 1 in magnitude (the others are below the pivot, so they do not count
+// for its ratio).  Ends with a CTA barrier.
+template <typename VT>
+__device__ __noinline__ void dense_panel(double* xj, double* ud, unsigned long long* vmax, int R, int w) {
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const int pw = (min(R, nt) + 31) >> 5;
+    auto scale = [](double v, double p, double rp) { return (double)ValTraits<VT>::to(div_by(v, p, rp)); };
+    auto sub = [](double a, double l, double u) { return __dsub_rn(a, __dmul_rn(l, u)); };
+    auto note = [&](int c, double v, double l) {
+        if (fabs(l) >= 1.0) atomicMax(vmax + c, (unsigned long long)__double_as_longlong(fabs(v)));
+    };
+    if (tid < 32) vmax[tid] = 0ull;
+    __syncthreads();
+    double x[32];
+    if (warp == 0) {
+        double* row = xj + (size_t)min(lane, R - 1) * 33;
+#pragma unroll
+        for (int c = 0; c < 32; c++) x[c] = lane < R ? row[c] : 0.0;
+#pragma unroll
+        for (int c = 0; c < 32; c++) {
+            if (c < w) {
+                constexpr int kAlign = ~3;
+                double* uc = ud + c * 34 - (c & kAlign);   // entry (c, q) at uc + q
+                if (lane == c) {
+#pragma unroll
+                    for (int q = c & kAlign; q < 32; q += 2) *(double2*)(uc + q) = make_double2(x[q], x[q + 1]);
+                }
+                const double p = __shfl_sync(0xffffffffu, x[c], c), rp = __drcp_rn(p);
+                if (lane == 0) ud[c * 34 + 32] = rp;
+                __syncwarp();
+                if (lane > c) {
+                    const double l = scale(x[c], p, rp);
+                    note(c, x[c], l);
+                    x[c] = l;
+                    if (!(c & 1)) x[c + 1] = sub(x[c + 1], l, uc[c + 1]);
+#pragma unroll
+                    for (int q = (c + 2) & ~1; q < 32; q += 2) {
+                        const double2 u = *(const double2*)(uc + q);
+                        x[q] = sub(x[q], l, u.x);
+                        x[q + 1] = sub(x[q + 1], l, u.y);
                     }
                 }
             }
-            lm = warp_max(lm);
-            if (lane == 0) wmax[c * 32 + warp] = lm;
-            __syncthreads();
+            if ((c & 3) == 3 && (c & ~3) < w && pw > 1) named_arrive(kBarPivots + (c >> 2), 32 * pw);
         }
+        __syncwarp();
+        if (lane < R) {
+#pragma unroll
+            for (int c = 0; c < 32; c++) row[c] = x[c];
+        }
+    }
+    for (int r0 = warp * 32 + (warp == 0 ? nt : 0); r0 < R; r0 += nt) {
+        const int r = r0 + lane;
+        double* row = xj + (size_t)min(r, R - 1) * 33;
+#pragma unroll
+        for (int c = 0; c < 32; c++) x[c] = r < R ? row[c] : 0.0;
+#pragma unroll 1
+        for (int c = 0; c < w; c += 4) {
+            const double* uc = ud + c * 34;
+            if (r0 < nt) named_sync(kBarPivots + (c >> 2), 32 * pw);
+            double v[4], l[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                v[k] = x[k];
+                l[k] = scale(x[k], uc[k * 34 + k], uc[k * 34 + 32]);
+#pragma unroll
+                for (int q = k + 1; q < 4; q++) x[q] = sub(x[q], l[k], uc[k * 34 + q]);
+            }
+#pragma unroll
+            for (int m = 4; m < 32; m += 4) {
+                if (m < 32 - c) {
+                    double y[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) y[q] = x[m + q];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const double2 e = *(const double2*)(uc + k * 34 + m);
+                        const double2 f = *(const double2*)(uc + k * 34 + m + 2);
+                        y[0] = sub(y[0], l[k], e.x);
+                        y[1] = sub(y[1], l[k], e.y);
+                        y[2] = sub(y[2], l[k], f.x);
+                        y[3] = sub(y[3], l[k], f.y);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; q++) x[m + q - 4] = y[q];
+                }
+            }
+            if (r < R) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) row[c + k] = l[k];
+            }
+            if (r < R && fmax(fmax(fabs(l[0]), fabs(l[1])), fmax(fabs(l[2]), fabs(l[3]))) >= 1.0) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) note(c + k, v[k], l[k]);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// The dense trailing block of one system (its own kernel: few warps, many
+// registers each): factor, VT storage for the solves (column-major, unit L
+// below the diagonal), inverses of its diagonal blocks, pivot statistics.
+template <typename VT, bool CL = false>
+__device__ void dense_phase(const SysDev& S, const SmemPlan& plan, char* smem_base, const SolveParams& prm) {
+    namespace cgr = cooperative_groups;
+    const PatternDev& P = *S.pat;
+    if (P.dtail <= 0) return;
+    Smem sm(smem_base, plan);
+    const int rank = CL ? (int)cgr::this_cluster().block_rank() : 0;
+    const int nranks = CL ? 2 : 1;
+    const int D = P.dtail, ld = P.tail_ld, k0 = P.k0, nbk = ld >> 5;
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    const int nup = nw - 1;                       // warps that update rows
+    double* xs = (double*)sm.uni;                 // [drows][33] the block column
+    double* ud = xs + (size_t)plan.drows * 33;     // [32][34] pivot rows of the panel
+    double* lk = ud;                              // [32][32] panel diagonal block (update phase)
+    double* ring = ud + 32 * 34;                  // [nup][dstg][4][32] panel rows in flight
+    unsigned long long* vmax = (unsigned long long*)ring;   // [32] column maxima (panel phase)
+    if (tid == 0) {
+        sm.ctl[1] = 0;
+        sm.ctl[2] = 0x7fffffff;
+        sm.ctl[3] = 0;
+        sm.ctl[kCtlPanels] = 0;
+    }
+    if (CL) cgr::this_cluster().sync();
+    else __syncthreads();
+    double* W = S.tailw;
+    VT* T = (VT*)S.tail;
+    double minpiv = INFINITY, minratio = INFINITY, maxu = 0.0;
+    int bad = 0;
+    long long c_panel = 0, c_update = 0, c_store = 0, tc = clock64();
+
+    for (int j = rank; j < nbk; j += nranks) {
+        const int w = min(32, D - 32 * j), R = D - 32 * j;
+        double* Wj = W + (size_t)j * D * 32;
+        // The block column from W, entries outside the pattern as 0.
+        for (int r0 = warp * 4; r0 < D; r0 += nw * 4) {
+            unsigned m[4];
+            double v[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) m[q] = r0 + q < D ? __ldg(P.tail_mask + (size_t)(r0 + q) * nbk + j) : 0u;
+#pragma unroll
+            for (int q = 0; q < 4; q++) v[q] = (m[q] >> lane) & 1u ? __ldcg(Wj + (size_t)(r0 + q) * 32 + lane) : 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (r0 + q < D) xs[(size_t)(r0 + q) * 33 + lane] = v[q];
+        }
+        __syncthreads();
+
+        // Panels 0 .. j - 1 applied in order.
+        if (warp == nup) {
+            for (int k = 0; k < j; k++) {
+                if (!dense_wait_panel(sm.ctl, k + 1, CL)) bad |= ST_WAIT_TIMEOUT;
+                const double* src = W + (size_t)k * D * 32 + (size_t)(32 * k) * 32;
+#pragma unroll 4
+                for (int t = lane; t < 512; t += 32) cp_async_16(lk + 2 * t, src + 2 * t);
+                // Rows of this U block updated by the panel before.
+                if (k > 0) named_sync(kBarRows, 32 * (min(8, nup) + 1));
+                cp_async_wait_all();
+                __syncwarp();
+                dense_solve_unit(lk, xs + (size_t)(32 * k) * 33 + lane);
+                named_arrive(kBarU, nt);
+            }
+        } else {
+            double* my = ring + (size_t)warp * plan.dstg * 128;
+            for (int k = 0; k < j; k++) {
+                if (!dense_wait_panel(sm.ctl, k + 1, CL)) bad |= ST_WAIT_TIMEOUT;
+                dense_update_rows(xs, xs + (size_t)(32 * k) * 33 + lane, W + (size_t)k * D * 32, my, 32 * (k + 1), D,
+                                  nup, plan.dstg, nt, k + 1 >= j || warp >= 8);
+            }
+        }
+        __syncthreads();
+        if (tid == 0) {
+            const long long t2 = clock64();
+            c_update += t2 - tc;
+            tc = t2;
+        }
+        double* xj = xs + (size_t)(32 * j) * 33;
+        dense_panel<VT>(xj, ud, vmax, R, w);
+        // Publish the panel: its rows to W, then the counters.
+        if (j + 1 < nbk) {
+            for (int t = tid; t < R * 32; t += nt) {
+                const int r = 32 * j + (t >> 5);
+                Wj[(size_t)r * 32 + lane] = xs[(size_t)r * 33 + lane];
+            }
+            __syncthreads();
+            if (tid == 0) {
+                share_fence(CL ? 2u : 1u);
+                *(volatile int*)(sm.ctl + kCtlPanels) = j + 1;
+                if (CL) *(volatile int*)cgr::this_cluster().map_shared_rank(sm.ctl + kCtlPanels, rank ^ 1) = j + 1;
+            }
+        }
+        if (tid == 0) {
+            const long long t2 = clock64();
+            c_panel += t2 - tc;
+            tc = t2;
+        }
+        // Off the chain: statistics, VT storage, inverses.
         if (tid < w) {
             const int c = tid;
-            const double piv = pan[c * ps + c];
+            const double piv = ud[c * 34 + (c & 3)];
             const double ap = fabs(piv);
-            double amax = 0.0;
-            for (int q = 0; q < nw; q++) amax = fmax(amax, wmax[c * 32 + q]);
+            const double amax = __longlong_as_double((long long)vmax[c]);
             if (!(ap > 0.0) || !isfinite(piv)) {
                 bad |= ST_SINGULAR;
-                atomicMin(&sm.ctl[2], k0 + jb + c);
+                atomicMin(&sm.ctl[2], k0 + 32 * j + c);
             }
             minpiv = fmin(minpiv, ap);
             const double ratio = amax > ap ? ap / amax : 1.0;
             minratio = fmin(minratio, ratio);
             if (ratio < prm.pivot_tol) bad |= ST_PIVOT_WEAK;
         }
-        for (int t = tid; t < R * nb; t += nt) {
-            const int r = t / nb, c = t - r * nb;
-            if (c < w) W[(size_t)(jb + r) * ld + jb + c] = pan[r * ps + c];
-        }
-        __syncthreads();
-    };
-    // A cluster factors panel 0 before the loop and each later panel one
-    // step ahead: rank 0 owns the next panel's 32 columns in the trailing
-    // update of the current step and factors that panel right after them,
-    // while rank 1 updates every other column (so the panel chain overlaps
-    // the bulk of the update).
-    if (CL && lead) panel(0);
-    for (int jb = 0; jb < D; jb += nb) {
-        const int w = min(nb, D - jb), R = D - jb;
-        const bool first = jb == 0;
-        if (!CL) panel(jb);
-        if (CL) {
-            // The panel is final in rank 0's shared memory and in W (first
-            // cluster barrier); rank 1 copies its multipliers, and rank 0
-            // overwrites them with the next panel only after the second
-            // (split: rank 0 arrives at once and waits just before that).
-            cluster_arrive();
-            cluster_wait();
-            if (!lead) {
-                const double* pan0 = cgr::this_cluster().map_shared_rank(pan, 0);
-                for (int t = tid; t < R * ps; t += nt) pan[t] = pan0[t];
-            }
-            cluster_arrive();
-            if (!lead) {
-                cluster_wait();
-                __syncthreads();
-            }
-        }
-        if (tid == 0) {
-            const long long t2 = clock64();
-            ctr[0] += t2 - ctr[3];
-            ctr[3] = t2;
-        }
-        const int c1 = jb + w, ncols = D - c1;
-        if (ncols <= 0) {
-            if (CL && lead) cluster_wait();
-            break;
-        }
-        // This CTA's columns of the trailing part, colof(t) the t-th: all of
-        // them, or (CL) the next panel's nb columns for rank 0 and the rest
-        // for rank 1.
-        const int cown = CL && !lead ? c1 + nb : c1;
-        const int nown = CL ? (lead ? min(nb, ncols) : max(0, ncols - nb)) : ncols;
-        const int cend = cown + nown;   // this CTA's columns: [cown, cend)
-        auto colof = [&](int t) { return cown + t; };
-        // U rows of the panel (triangular solve with the unit-L diagonal
-        // block), one thread per column, in groups of 8 rows so the column
-        // stays in registers.
-        for (int t = tid; t < nown; t += nt) {
-            const int colc = colof(t);
-            if (colc >= cend) continue;
-            const size_t col = (size_t)colc;
-            for (int g = 0; g < w; g += 8) {
-                double u[8];
-#pragma unroll
-                for (int r = 0; r < 8; r++) u[r] = g + r < w ? tail_entry<CL>(W, ld, mask, jb + g + r, (int)col, first) : 0.0;
-                for (int g2 = 0; g2 < g; g2 += 8) {
-                    double v[8];
-#pragma unroll
-                    for (int c = 0; c < 8; c++) v[c] = wld((size_t)(jb + g2 + c) * ld + col);
-#pragma unroll
-                    for (int c = 0; c < 8; c++)
-#pragma unroll
-                        for (int r = 0; r < 8; r++)
-                            if (g + r < w) u[r] = __dsub_rn(u[r], __dmul_rn(pan[(g + r) * ps + g2 + c], v[c]));
-                }
-#pragma unroll
-                for (int c = 0; c < 8; c++)
-#pragma unroll
-                    for (int r = c + 1; r < 8; r++)
-                        if (g + r < w) u[r] = __dsub_rn(u[r], __dmul_rn(pan[(g + r) * ps + g + c], u[c]));
-#pragma unroll
-                for (int r = 0; r < 8; r++)
-                    if (g + r < w) W[(size_t)(jb + g + r) * ld + col] = u[r];
+        for (int c = warp; c < w; c += nw) {
+            const int col = 32 * j + c;
+            for (int i = lane; i < ld; i += 32) {
+                const double v = i < D ? xs[(size_t)i * 33 + c] : 0.0;
+                if (i <= col) maxu = fmax(maxu, fabs(v));
+                T[(size_t)col * ld + i] = ValTraits<VT>::to(v);
             }
         }
         __syncthreads();
         if (tid == 0) {
             const long long t2 = clock64();
-            ctr[1] += t2 - ctr[3];
-            ctr[3] = t2;
-        }
-        // Trailing update W22 -= L21 U12, tiles of (4 * nw) rows x 128
-        // columns: a thread owns four rows (one per warp stride) and four
-        // columns (lane + 32 j); multipliers from the panel in shared memory
-        // (broadcast within a warp), U12 staged per tile.
-        if (CL && lead) {
-            // Rank 0's single panel-wide chunk (at most 32 columns): tiles
-            // of 16 nw rows x 32 columns, a thread owning one column and 16
-            // rows (one per warp stride), so no lane idles.
-            const int TRn = 16 * nw;
-            for (int r0 = c1; r0 < D; r0 += TRn) {
-                for (int t = tid; t < w * 32; t += nt) {
-                    const int c = t >> 5, x = t & 31;
-                    const int col = cown + x;
-                    ut[c * 128 + x] = col < cend ? wld((size_t)(jb + c) * ld + col) : 0.0;
-                }
-                __syncthreads();
-                const int rw = r0 + warp, col = cown + lane;
-                if (rw < D) {
-                    double acc[16];
-                    int lo[16];
-#pragma unroll
-                    for (int k = 0; k < 16; k++) {
-                        const int row = rw + k * nw;
-                        lo[k] = row < D ? k * nw * ps : 0;   // rows past the block reuse rw's multipliers
-                        acc[k] = (row < D && col < cend) ? tail_entry<CL>(W, ld, mask, row, col, first) : 0.0;
-                    }
-                    const double* l0 = pan + (size_t)(rw - jb) * ps;
-                    for (int c = 0; c < w; c++) {
-                        const double u = ut[c * 128 + lane];
-#pragma unroll
-                        for (int k = 0; k < 16; k++) acc[k] = __dsub_rn(acc[k], __dmul_rn(l0[lo[k] + c], u));
-                    }
-#pragma unroll
-                    for (int k = 0; k < 16; k++) {
-                        const int row = rw + k * nw;
-                        if (row < D && col < cend) W[(size_t)row * ld + col] = acc[k];
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        const int TR = 4 * nw;
-        const int nrt = (ncols + TR - 1) / TR, nct = CL && lead ? 0 : (nown + 127) / 128;
-        for (int tile = 0; tile < nrt * nct; tile++) {
-            const int r0 = c1 + (tile / nct) * TR, tq = (tile % nct) * 128;
-            for (int t = tid; t < w * 128; t += nt) {
-                const int c = t >> 7, x = t & 127;
-                const int col = colof(tq + x);
-                ut[t] = col < cend ? wld((size_t)(jb + c) * ld + col) : 0.0;
-            }
-            __syncthreads();
-            const int rw = r0 + warp;
-            if (rw < D) {
-                double acc[4][4];
-                int lo[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int row = rw + q * nw;
-                    lo[q] = row < D ? q * nw * ps : 0;   // rows past the block reuse rw's multipliers
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int col = colof(tq + lane + 32 * j);
-                        acc[q][j] = (row < D && col < cend) ? tail_entry<CL>(W, ld, mask, row, col, first) : 0.0;
-                    }
-                }
-                const double* l0 = pan + (size_t)(rw - jb) * ps;
-                for (int c = 0; c < w; c++) {
-                    double u[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j++) u[j] = ut[c * 128 + lane + 32 * j];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const double l = l0[lo[q] + c];
-#pragma unroll
-                        for (int j = 0; j < 4; j++) acc[q][j] = __dsub_rn(acc[q][j], __dmul_rn(l, u[j]));
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int row = rw + q * nw;
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int col = colof(tq + lane + 32 * j);
-                        if (row < D && col < cend) W[(size_t)row * ld + col] = acc[q][j];
-                    }
-                }
-            }
-            __syncthreads();
-        }
-        if (tid == 0) {
-            const long long t2 = clock64();
-            ctr[2] += t2 - ctr[3];
-            ctr[3] = t2;
-        }
-        if (CL && lead) {
-            // The next panel's columns are final (this CTA's own update):
-            // make them visible at L2, where the panel load reads; rank 1
-            // is done copying this panel.
-            __threadfence();
-            __syncthreads();
-            cluster_wait();
-            panel(c1);
-            if (tid == 0) {
-                const long long t2 = clock64();
-                ctr[0] += t2 - ctr[3];
-                ctr[3] = t2;
-            }
+            c_store += t2 - tc;
+            tc = t2;
         }
     }
-    if (tid == 0 && lead) {
-        st->cyc_tpanel = ctr[0];
-        st->cyc_ttrsm = ctr[1];
-        st->cyc_tupdate = ctr[2];
-    }
-}
-
-// Dense trailing block -> VT storage for the solves (unit L below the
-// diagonal, U on and above).  The block's entries live only there (the
-// merged slot array gets them from merge_factor_kernel when a caller asks).
-template <typename VT, bool CG = false>
-__device__ void dense_tail_store(const SysDev& S, const PatternDev& P, const double* W, double& maxu,
-                                 char* smem_tail_tiles, int ttw) {
-    const int D = P.dtail, ld = P.tail_ld, k0 = P.k0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    VT* T = (VT*)S.tail;
-    // T is column-major (element (i, c) at T[c * ld + i]) so the solves'
-    // block-column products read consecutive rows per warp.  Transpose in
-    // 32 x 32 tiles through shared memory (a warp per tile, ttw warps,
-    // each with a padded 32 x 33 fp64 tile).
-    {
-        double* tile = (double*)smem_tail_tiles + (size_t)warp * 32 * 33;
-        const int nt32 = ld / 32, twarps = min(nw, ttw);
-        if (warp < twarps) {
-            for (int tt = warp; tt < nt32 * nt32; tt += twarps) {
-                const int ti = tt / nt32, tc = tt - ti * nt32;
-                for (int r = 0; r < 32; r++) {
-                    const int i = ti * 32 + r, c = tc * 32 + lane;
-                    double v = 0.0;
-                    if (i < D && c < D) {
-                        v = CG ? __ldcg(W + (size_t)i * ld + c) : W[(size_t)i * ld + c];
-                        if (i <= c) maxu = fmax(maxu, fabs(v));
-                    }
-                    tile[r * 33 + lane] = v;
-                }
-                __syncwarp();
-                for (int c = 0; c < 32 && tc * 32 + c < D; c++)
-                    T[(size_t)(tc * 32 + c) * ld + ti * 32 + lane] = ValTraits<VT>::to(tile[lane * 33 + c]);
-                __syncwarp();
+    // Inverses of the diagonal blocks, once every block column is stored: a
+    // warp per block and factor, over both CTAs of a cluster.  The factors
+    // are read as the solves read them (VT-rounded): unit L and, rows and
+    // columns reversed, U are two lower triangles; the identity past a
+    // partial block.  Element (i, c) of an inverse at c * 32 + i.
+    if (CL) cgr::this_cluster().sync();
+    const int ntile = min(nw, (int)((plan.bytes - (size_t)((char*)xs - smem_base)) / (32 * 34 * sizeof(double))));
+    if (warp < ntile) {
+        double* bs = xs + (size_t)warp * 32 * 34;   // [32][34], reciprocal diagonal in column 32
+        for (int task = rank + nranks * warp; task < 2 * nbk; task += nranks * ntile) {
+            const int j = task >> 1, up = task & 1, w = min(32, D - 32 * j);
+            const VT* blk = T + (size_t)(32 * j) * ld + 32 * j;
+            // Column by column (contiguous in T): lane = row.
+            const int r = up ? 31 - lane : lane;
+            double dg = 1.0;
+#pragma unroll 8
+            for (int cc = 0; cc < 32; cc++) {
+                const bool in = lane < w && cc < w && (up || lane != cc);
+                double v = lane == cc ? 1.0 : 0.0;
+                if (in) v = ValTraits<VT>::load_cg(blk + (size_t)cc * ld + lane);
+                const int c = up ? 31 - cc : cc;
+                if (c <= r) bs[r * 34 + c] = v;
+                if (c == r) dg = v;
             }
-        }
-    }
-    __syncthreads();
-    (void)k0;
-}
-
-// The dense trailing block of one system (its own kernel: few warps, many
-// registers each): factor, store, merge the pivot statistics.
-// Inverses of the 32 x 32 diagonal blocks of the dense block's factor, for
-// the solves (a block's triangular solve becomes a matrix-vector product
-// instead of a 32-step dependent chain), from the factored fp64 block W
-// rounded to VT exactly as the stored factor is: a warp per block and
-// factor (nwork warps, each with a 32 x 33 block tile and a 32 x 33 tile of
-// the inverse at work + warp * 2 * 32 * 33 doubles), lane c computing column
-// c in fp64 by substitution; stored as VT with element (i, c) at c * 32 + i.
-// Rows and columns past a partial last block are the identity.  W read
-// through L2 (another CTA of a cluster may have written it).
-template <typename VT>
-__device__ void dense_tail_inverses(const SysDev& S, const PatternDev& P, double* work, int nwork) {
-    const int D = P.dtail, ld = P.tail_ld;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double* W = S.tailw;
-    VT* out = (VT*)S.tinv;
-    const int nbk = (D + 31) / 32;
-    double* Bs = work + (size_t)warp * 2 * 32 * 33;   // block: row r at r * 33
-    double* Xs = Bs + 32 * 33;                        // inverse: X[k][c] at k * 33 + c
-    if (warp < nwork) {
-        for (int task = warp; task < 2 * nbk; task += nwork) {
-            const int b = task >> 1, upper = task & 1, jb = b * 32, w = min(32, D - jb);
-            for (int r = 0; r < 32; r++)
-                Bs[r * 33 + lane] = (r < w && lane < w)
-                                        ? (double)ValTraits<VT>::to(__ldcg(W + (size_t)(jb + r) * ld + jb + lane))
-                                        : 0.0;
+            bs[r * 34 + 32] = __drcp_rn(dg);
             __syncwarp();
-            const int c = lane;
-            if (!upper) {
-                // X = L^-1 (unit lower): X[r][c] = -sum_{c<=k<r} L[r][k] X[k][c].
-                for (int r = 0; r < 32; r++) {
-                    double s0 = 0.0, s1 = 0.0;
-                    int k = 0;
-                    for (; k + 1 < r; k += 2) {
-                        s0 = fma(Bs[r * 33 + k], Xs[k * 33 + c], s0);
-                        s1 = fma(Bs[r * 33 + k + 1], Xs[(k + 1) * 33 + c], s1);
-                    }
-                    if (k < r) s0 = fma(Bs[r * 33 + k], Xs[k * 33 + c], s0);
-                    Xs[r * 33 + c] = r < c ? 0.0 : r == c ? 1.0 : r >= w ? 0.0 : -(s0 + s1);
-                    __syncwarp();
-                }
-            } else {
-                // X = U^-1: X[r][c] = -(sum_{r<k<=c} U[r][k] X[k][c]) / U[r][r].
-                for (int r = 31; r >= 0; r--) {
-                    double s0 = 0.0, s1 = 0.0;
-                    int k = r + 1;
-                    for (; k + 1 < 32; k += 2) {
-                        s0 = fma(Bs[r * 33 + k], Xs[k * 33 + c], s0);
-                        s1 = fma(Bs[r * 33 + k + 1], Xs[(k + 1) * 33 + c], s1);
-                    }
-                    if (k < 32) s0 = fma(Bs[r * 33 + k], Xs[k * 33 + c], s0);
-                    const double dg = r < w ? Bs[r * 33 + r] : 1.0;
-                    Xs[r * 33 + c] = r > c ? 0.0 : r == c ? 1.0 / dg : r >= w ? 0.0 : -(s0 + s1) / dg;
-                    __syncwarp();
-                }
-            }
-            VT* dst = out + (size_t)b * 2048 + (size_t)upper * 1024;
-            for (int cc = 0; cc < 32; cc++) dst[cc * 32 + lane] = ValTraits<VT>::to(Xs[lane * 33 + cc]);
+            VT* inv = (VT*)S.tinv + (size_t)j * 2048 + up * 1024;
+            if (!up) dense_block_inverse<VT>(bs, inv + lane * 32, 1);
+            else dense_block_inverse<VT>(bs, inv + (31 - lane) * 32 + 31, -1);
             __syncwarp();
         }
     }
-}
-
-// CL: the two CTAs of a thread-block cluster share the system (see
-// dense_tail_factor); rank 0 stores the factor and the statistics.
-template <typename VT, bool CL = false>
-__device__ void dense_phase(const SysDev& S, const SmemPlan& plan, char* smem_base, const SolveParams& prm) {
-    const PatternDev& P = *S.pat;
-    if (P.dtail <= 0) return;
-    Smem sm(smem_base, plan);
-    if (threadIdx.x == 0) {
-        sm.ctl[1] = 0;
-        sm.ctl[2] = 0x7fffffff;
+    // Statistics: rank 0 merges, then rank 1; the cluster barriers also keep
+    // each CTA's shared memory alive until the other is done with it.
+    for (int r = 0; r < nranks; r++) {
+        if (rank == r) cta_store_pivot_stats(S.stats, sm, minpiv, minratio, maxu, bad, false, sm.ctl);
+        if (CL) cgr::this_cluster().sync();
     }
-    __syncthreads();
-    double minpiv = INFINITY, minratio = INFINITY, maxu = 0.0;
-    int bad = 0;
-    dense_tail_factor<VT, CL>(P, S.tailw, sm, plan, prm, minpiv, minratio, bad, S.stats);
-    __syncthreads();
-    // Warps that fit a block tile and an inverse tile in this CTA's area.
-    const size_t uoff = (size_t)(sm.uni - smem_base);
-    const int nwork = (int)min((size_t)(blockDim.x >> 5),
-                               (plan.bytes > uoff ? plan.bytes - uoff : 0) / (2 * 32 * 33 * sizeof(double)));
-    if (CL && cooperative_groups::this_cluster().block_rank() != 0) {
-        // Rank 1 computes the inverses while rank 0 stores the factor.
-        dense_tail_inverses<VT>(S, P, (double*)sm.uni, nwork);
-        return;
+    if (tid == 0 && rank == 0) {
+        S.stats->cyc_tpanel = c_panel;
+        S.stats->cyc_ttrsm = c_store;
+        S.stats->cyc_tupdate = c_update;
     }
-    dense_tail_store<VT, CL>(S, P, S.tailw, maxu, sm.uni, plan.ttw);
-    if (!CL) dense_tail_inverses<VT>(S, P, (double*)sm.uni, nwork);
-    cta_store_pivot_stats(S.stats, sm, minpiv, minratio, maxu, bad, false, sm.ctl);
 }
 
 // ---------------------------------------------------------------------------
@@ -610,11 +647,6 @@ __device__ void dense_phase(const SysDev& S, const SmemPlan& plan, char* smem_ba
 // Shared memory per warp: x[wcap] (fp64), a stage of scap L values (VT) and
 // scap + 16 relative slots.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async_16(void* sdst, const void* gsrc) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
-}
-
 // Spread mode: the pivot statistics and cycle counters of one CTA merged
 // into the system's sync area; the last CTA to finish writes the system's
 // statistics (pivot minima through the bit patterns of non-negative doubles:
@@ -980,7 +1012,7 @@ __device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem
                         maxu = fmax(maxu, fabs(v));
                         uval[dst[q]] = ValTraits<VT>::to(v);
                     } else {
-                        W[(size_t)(dst[q] - P.k0) * P.tail_ld + (k - P.k0)] = v;
+                        W[tail_index(P.dtail, dst[q] - P.k0, k - P.k0)] = v;
                     }
                 }
             }
@@ -1005,6 +1037,7 @@ __device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem
         const double ratio = amax > ap ? ap / amax : 1.0;
         minratio = fmin(minratio, ratio);
         if (ratio < prm.pivot_tol) bad |= ST_PIVOT_WEAK;
+        const double rpiv = __drcp_rn(piv);
         // Each value is stored once where the solves read it (U rows, the
         // diagonal, L rows); the strict-L part also goes to the merged
         // columns, which the later columns' gathers read.  The destinations
@@ -1022,13 +1055,13 @@ __device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem
                 const int t = t0 + 32 * q;
                 if (t >= len) break;
                 double v = x[t];
-                if (t > d) v = __ddiv_rn(v, piv);
+                if (t > d) v = div_by(v, piv, rpiv);
                 else maxu = fmax(maxu, fabs(v));
                 const VT sv = ValTraits<VT>::to(v);
                 if (t < d) uval[dst[q]] = sv;
                 else if (t == d) {
                     udiag[k] = sv;
-                    ((VT*)S.udiag_bwd)[bpos] = ValTraits<VT>::to(1.0 / piv);
+                    ((VT*)S.udiag_bwd)[bpos] = ValTraits<VT>::to(rpiv);
                 } else {
                     lu[c0 + t] = sv;
                     lval[dst[q]] = sv;
