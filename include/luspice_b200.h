@@ -121,10 +121,10 @@ typedef struct {
                                       ready bits), 2 level-synchronous (barrier per
                                       level; descriptors in shared memory when they
                                       fit, else read from global memory) */
-    int refactor_mode;             /* gathers of dependency columns: 0 staged in
-                                      shared memory by asynchronous copies with
-                                      precomputed relative slots, 1 loaded per
-                                      dependency with a search of the column's rows */
+    int refactor_mode;             /* updates from dependency columns: 0 by segments of
+                                      consecutive columns of one supernode with
+                                      precomputed relative slots, 1 per dependency
+                                      with a search of the column's rows */
     int inner_prec;                /* A in the inner GMRES products (mixed path):
                                       0 fp32 values (default), 1 fp64 values (first
                                       escalation step for ill-conditioned systems),

@@ -152,6 +152,7 @@ __device__ __forceinline__ double block_min(double v, double* scratch) {
 // its sign.  Why: a dependent chain of 40 cycles after the reciprocal (61);
 // __ddiv_rn takes 420 for a warp with one zero dividend (measured, B200).
 static __device__ __noinline__ double div_call(double a, double b) { return __ddiv_rn(a, b); }
+template <bool CALL = true>
 __device__ __forceinline__ double div_by(double a, double b, double rb) {
     const double q0 = __dmul_rn(a, rb);
     const double q1 = fma(fma(-b, q0, a), rb, q0);
@@ -160,7 +161,7 @@ __device__ __forceinline__ double div_by(double a, double b, double rb) {
     const bool in = eb - 623u <= 800u;
     if (in && ea - 623u <= 800u) return q2;
     if (in && a == 0.0) return q0;
-    return div_call(a, b);   // a call: the expansion stays out of unrolled loops
+    return CALL ? div_call(a, b) : __ddiv_rn(a, b);   // a call keeps the expansion out of unrolled loops
 }
 
 template <typename T> struct ValTraits;

@@ -66,10 +66,11 @@ __global__ void __launch_bounds__(MAXT, 1)
 refactor_kernel(const SysDev* __restrict__ sys, int nsys, int* queue, SmemPlan plan, SolveParams prm,
                 const int* dyn, const int* list, SpreadArgs sp) {
     extern __shared__ __align__(16) char smem[];
+    __shared__ RefactorCtx cx;
     __shared__ int s_task;
     const int ns = item_count(nsys, dyn);
     (void)sp;
-    // A thread-block cluster (or a lone CTA) takes one system at a time:
+    // A thread-block cluster takes one system at a time:
     // rank 0 draws it, every CTA reads it through distributed shared memory
     // between two cluster barriers (so rank 0 outlives the read).
     namespace cgr = cooperative_groups;
@@ -82,8 +83,30 @@ refactor_kernel(const SysDev* __restrict__ sys, int nsys, int* queue, SmemPlan p
         const int t = *task0;
         cl.sync();
         if (t >= ns) break;
-        const SysDev S = sys[list ? list[t] : t];
-        refactor_phase<VT>(S, plan, smem, prm);
+        load_ctx(cx, sys + (list ? list[t] : t));
+        refactor_phase<VT>(cx, plan, smem, prm);
+    }
+}
+
+// One CTA per system, without a cluster: claims, ready bits and factor values
+// stay in the CTA's shared memory and its SM's L1.
+template <typename VT, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+refactor_lone_kernel(const SysDev* __restrict__ sys, int nsys, int* queue, SmemPlan plan, SolveParams prm,
+                     const int* dyn, const int* list, SpreadArgs sp) {
+    extern __shared__ __align__(16) char smem[];
+    __shared__ RefactorCtx cx;
+    __shared__ int s_task;
+    const int ns = item_count(nsys, dyn);
+    (void)sp;
+    while (true) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_task = atomicAdd(queue, 1);
+        __syncthreads();
+        const int t = s_task;
+        if (t >= ns) break;
+        load_ctx(cx, sys + (list ? list[t] : t));
+        refactor_phase<VT, false, true>(cx, plan, smem, prm);
     }
 }
 
@@ -99,8 +122,9 @@ refactor_spread_kernel(const SysDev* __restrict__ sys, int nsys, int* queue, Sme
     const int ns = item_count(nsys, dyn);
     const int t = (int)blockIdx.x / sp.group;
     if (t >= ns) return;
-    const SysDev S = sys[list ? list[t] : t];
-    refactor_phase<VT, true>(S, plan, smem, prm, sp.sync + (size_t)t * sp.stride, (int)blockIdx.x % sp.group,
+    __shared__ RefactorCtx cx;
+    load_ctx(cx, sys + (list ? list[t] : t));
+    refactor_phase<VT, true>(cx, plan, smem, prm, sp.sync + (size_t)t * sp.stride, (int)blockIdx.x % sp.group,
                              sp.group);
 }
 
@@ -316,10 +340,10 @@ int pattern_build(int n, const int* Ap, const int* Ai, const double* Ax, const i
     build_static_pattern(n, Ap, Ai, q.data(), F, 256, P->S, dense_tail);
     const StaticPattern& S = P->S;
     // Column records of the refactorization (see PatternDev::crec).
-    std::vector<int> crec((size_t)12 * n, 0);
+    std::vector<int> crec((size_t)16 * n, 0);
     for (int idx = 0; idx < n; idx++) {
         const int k = S.col_order[idx];
-        int* r = crec.data() + (size_t)12 * idx;
+        int* r = crec.data() + (size_t)16 * idx;
         const int c0 = S.cp[k], d = S.dg[k] - c0;
         int dsp = d;
         if (k >= S.k0) {
@@ -338,6 +362,9 @@ int pattern_build(int n, const int* Ap, const int* Ai, const double* Ax, const i
         r[8] = (int)(unsigned)(rp & 0xffffffffll);
         r[9] = (int)(unsigned)((unsigned long long)rp >> 32);
         r[10] = S.a_diag[k];
+        r[12] = S.seg_ptr.empty() ? 0 : S.seg_ptr[k];
+        r[13] = S.seg_ptr.empty() ? 0 : S.seg_ptr[k + 1] - S.seg_ptr[k];
+        r[14] = S.lp[k];
     }
     // Bit pattern of the dense trailing block (see PatternDev::tail_mask).
     std::vector<int> tail_mask;
@@ -358,7 +385,7 @@ int pattern_build(int n, const int* Ap, const int* Ai, const double* Ax, const i
                                         &S.lrp, &S.lci, &S.urp, &S.uci, &S.slot_dst, &S.fwd_order,
                                         &S.bwd_order, &S.sell_ptr, &S.sell_col, &S.sell_src,
                                         &S.sell_perm, &S.rowat, &S.q, &S.fwd_lev, &S.bwd_lev, &S.bwd_pos,
-                                        &S.fwd_ldesc, &S.bwd_ldesc, &S.dep_bc, &S.a_diag, &tail_mask, &crec};
+                                        &S.fwd_ldesc, &S.bwd_ldesc, &S.lp, &S.seg, &S.a_diag, &tail_mask, &crec};
     const int narr = (int)(sizeof(arrays) / sizeof(arrays[0]));
     std::vector<size_t> off(narr + 1, 0);
     // Each array gets at least 8 ints of slack: the sweeps copy index runs
@@ -380,6 +407,7 @@ int pattern_build(int n, const int* Ap, const int* Ai, const double* Ax, const i
     D.max_col = S.max_col;
     D.nslices = S.nslices;
     D.sell_total = S.sell_ptr.empty() ? 0 : S.sell_ptr.back();
+    D.nnz_lcol = S.lp[S.k0];
     D.nnz_l = (int)S.lci.size();
     D.nnz_u = (int)S.uci.size();
     int idx = 0;
@@ -408,7 +436,9 @@ int pattern_build(int n, const int* Ap, const int* Ai, const double* Ax, const i
     D.bwd_pos = blk + off[idx++];
     D.fwd_ldesc = blk + off[idx++];
     D.bwd_ldesc = blk + off[idx++];
-    D.dep_bc = (const int2*)(blk + off[idx++]);
+    D.lp = blk + off[idx++];
+    D.seg = S.seg_ptr.empty() ? nullptr : (const int4*)(blk + off[idx]);
+    idx++;
     D.a_diag = blk + off[idx++];
     D.tail_mask = S.dtail > 0 ? (const unsigned*)(blk + off[idx]) : nullptr;
     idx++;
@@ -420,24 +450,16 @@ int pattern_build(int n, const int* Ap, const int* Ai, const double* Ax, const i
     D.k0 = S.k0;
     D.dtail = S.dtail;
     D.tail_ld = tail_ld(S);
-    // Relative update slots: rel_ptr (n+1 int64) then rel (16 bit, padded by
-    // 16 entries so aligned 16-byte copies never run past the end).
+    // Relative update slots (column records hold their offsets).
     D.rel = nullptr;
-    D.rel_ptr = nullptr;
     if (!S.rel_ptr.empty()) {
-        const size_t pbytes = ((S.rel_ptr.size() * sizeof(long long)) + 255) & ~(size_t)255;
-        const size_t rbytes = (S.rel.size() + 16) * sizeof(uint16_t);
-        e = cudaMalloc(&P->d_rel, pbytes + rbytes);
+        const size_t rbytes = (S.rel.size() + 1) * sizeof(uint16_t);
+        e = cudaMalloc(&P->d_rel, rbytes);
         if (e != cudaSuccess) { pattern_free(P); return cuda_fail(e, "pattern rel alloc"); }
-        char* rb = (char*)P->d_rel;
-        e = cudaMemcpy(rb, S.rel_ptr.data(), S.rel_ptr.size() * sizeof(long long), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && !S.rel.empty())
-            e = cudaMemcpy(rb + pbytes, S.rel.data(), S.rel.size() * sizeof(uint16_t), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemset(rb + pbytes + S.rel.size() * sizeof(uint16_t), 0, 16 * sizeof(uint16_t));
+        if (!S.rel.empty()) e = cudaMemcpy(P->d_rel, S.rel.data(), S.rel.size() * sizeof(uint16_t), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) { pattern_free(P); return cuda_fail(e, "pattern rel upload"); }
-        D.rel_ptr = (const long long*)rb;
-        D.rel = (const unsigned short*)(rb + pbytes);
-        P->bytes += pbytes + rbytes;
+        D.rel = (const unsigned short*)P->d_rel;
+        P->bytes += rbytes;
     }
     e = cudaMalloc(&P->d_desc, sizeof(PatternDev));
     if (e != cudaSuccess) { pattern_free(P); return cuda_fail(e, "pattern descriptor alloc"); }
@@ -491,7 +513,6 @@ void make_plan(const std::vector<PatternObj*>& pats, int block, int ctas_per_sm,
     plan.nwords = (nmax + 31) / 32;
     plan.m = m;
     plan.wcap = 0;
-    plan.scap = 0;
     const size_t fixed = smem_fixed(plan.nwords);
     const size_t hbytes = ((size_t)(m + 1) * m + 6 * (size_t)(m + 1)) * sizeof(double);
     size_t avail = budget > fixed + hbytes ? budget - fixed - hbytes : 0;
@@ -554,24 +575,14 @@ void make_refactor_plan(const std::vector<PatternObj*>& pats, int threads, int v
     plan.ycap = 0;
     plan.dcap = 0;
     const size_t fixed = smem_fixed(plan.nwords);
+    budget -= sizeof(RefactorCtx) + 256;   // static shared memory of the kernels
     const int nw = threads / 32;
     const size_t per_warp = budget > fixed ? (budget - fixed) / nw : 0;
-    // Per warp: work vector (wcap fp64), stage of scap values and scap + 16
-    // relative slots.  Prefer the whole longest column in shared memory,
-    // then the largest stage (512 down to 64 entries).
-    auto need = [&](int wcap, int scap) {
-        return (size_t)wcap * 8 + (size_t)scap * vsize + ((size_t)scap + 16) * 2;
-    };
-    int scap = 512;
-    while (scap > 64 && need(colmax, scap) > per_warp) scap /= 2;
-    int wcap = colmax;
-    if (need(wcap, scap) > per_warp) {
-        const size_t rest = per_warp > need(0, scap) ? per_warp - need(0, scap) : 0;
-        wcap = (int)std::min<size_t>((size_t)colmax, rest / 8) & ~1;
-    }
-    plan.wcap = wcap;
-    plan.scap = scap;
-    plan.bytes = fixed + (size_t)nw * need(wcap, scap);
+    // Per warp: its column's record and pivot minima, and a work vector (wcap
+    // fp64), the longest column when it fits.
+    (void)vsize;
+    plan.wcap = (int)std::min<size_t>((size_t)colmax, per_warp > kWarpHead ? (per_warp - kWarpHead) / 8 : 0) & ~1;
+    plan.bytes = fixed + (size_t)nw * (plan.wcap * 8 + kWarpHead);
 }
 
 void make_dense_plan(const std::vector<PatternObj*>& pats, int threads, SmemPlan& plan) {
@@ -628,30 +639,35 @@ static int kernel_prepare(size_t smem, int block, int* occ) {
 
 using RefactorFn = void (*)(const SysDev*, int, int*, SmemPlan, SolveParams, const int*, const int*, SpreadArgs);
 
+// How a system's refactorization is shared: by a thread-block cluster, by
+// one CTA, or by CTAs anywhere on the GPU.
+enum RefactorKind { kCluster = 0, kLone = 1, kSpread = 2 };
+
 // The refactor instance for a CTA of block threads: one CTA per SM above
 // 512 threads (the instance with the most registers that still fits the
 // block), else the 1024-thread instance, whose CTAs pack several per SM.
 template <typename VT>
-static RefactorFn refactor_fn(int block, bool spread = false) {
-    if (spread) return block <= 512 ? refactor_spread_kernel<VT, 1024> : refactor_spread_kernel<VT, 768>;
-    if (block <= 512) return refactor_kernel<VT, 1024>;
-    if (block <= 640) return refactor_kernel<VT, 640>;
-    if (block <= 768) return refactor_kernel<VT, 768>;
-    return refactor_kernel<VT, 1024>;
+static RefactorFn refactor_fn(int block, RefactorKind kind, int* slot = nullptr) {
+    const int size = block <= 512 ? 0 : block <= 640 && kind == kCluster ? 1 : block <= 768 ? 2 : 0;
+    if (slot) *slot = kind * 3 + size;
+    if (kind == kSpread) return size == 0 ? refactor_spread_kernel<VT, 1024> : refactor_spread_kernel<VT, 768>;
+    if (kind == kLone) return size == 0 ? refactor_lone_kernel<VT, 1024> : refactor_lone_kernel<VT, 768>;
+    return size == 0 ? refactor_kernel<VT, 1024> : size == 1 ? refactor_kernel<VT, 640> : refactor_kernel<VT, 768>;
 }
 
 template <typename VT>
-static int refactor_prepare(size_t smem, int block, int* occ, bool spread = false) {
+static int refactor_prepare(size_t smem, int block, int* occ, RefactorKind kind) {
     static std::mutex mu;
-    static size_t granted[5] = {0, 0, 0, 0, 0};   // per instance: 1024, 640, 768, spread 1024, spread 768
-    const int slot = spread ? (block <= 512 ? 3 : 4) : block <= 512 || block > 768 ? 0 : block <= 640 ? 1 : 2;
-    return prepare_kernel(refactor_fn<VT>(block, spread), smem, block, occ, &granted[slot], mu);
+    static size_t granted[9] = {};   // per instance
+    int slot = 0;
+    const RefactorFn fn = refactor_fn<VT>(block, kind, &slot);
+    return prepare_kernel(fn, smem, block, occ, &granted[slot], mu);
 }
 
 // Clusters of csize refactor CTAs that can be resident at once.
 template <typename VT>
 static int refactor_cluster_count(size_t smem, int block, int csize, int* nclusters) {
-    int rc = refactor_prepare<VT>(smem, block, nullptr);
+    int rc = refactor_prepare<VT>(smem, block, nullptr, kCluster);
     if (rc != LUSP_OK) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)csize * sm_count());
@@ -664,7 +680,7 @@ static int refactor_cluster_count(size_t smem, int block, int csize, int* nclust
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaOccupancyMaxActiveClusters(nclusters, refactor_fn<VT>(block), &cfg);
+    cudaError_t e = cudaOccupancyMaxActiveClusters(nclusters, refactor_fn<VT>(block, kCluster), &cfg);
     if (e != cudaSuccess) return cuda_fail(e, "cluster occupancy query");
     return LUSP_OK;
 }
@@ -703,11 +719,14 @@ static int dense_cluster_count(size_t smem, int block, int* nclusters) {
 // the serving loop pays that once at creation instead of inside a request).
 int preload_kernels() {
     const void* fns[] = {
-        (const void*)refactor_fn<float>(512), (const void*)refactor_fn<float>(640), (const void*)refactor_fn<float>(768),
-        (const void*)refactor_fn<double>(512), (const void*)refactor_fn<double>(640),
-        (const void*)refactor_fn<double>(768), (const void*)refactor_fn<float>(768, true),
-        (const void*)refactor_fn<float>(512, true), (const void*)refactor_fn<double>(768, true),
-        (const void*)refactor_fn<double>(512, true), (const void*)dense_kernel<float>, (const void*)dense_kernel<double>,
+        (const void*)refactor_fn<float>(512, kCluster), (const void*)refactor_fn<float>(640, kCluster),
+        (const void*)refactor_fn<float>(768, kCluster), (const void*)refactor_fn<double>(512, kCluster),
+        (const void*)refactor_fn<double>(640, kCluster), (const void*)refactor_fn<double>(768, kCluster),
+        (const void*)refactor_fn<float>(512, kLone), (const void*)refactor_fn<float>(768, kLone),
+        (const void*)refactor_fn<double>(512, kLone), (const void*)refactor_fn<double>(768, kLone),
+        (const void*)refactor_fn<float>(512, kSpread), (const void*)refactor_fn<float>(768, kSpread),
+        (const void*)refactor_fn<double>(512, kSpread), (const void*)refactor_fn<double>(768, kSpread),
+        (const void*)dense_kernel<float>, (const void*)dense_kernel<double>,
         (const void*)dense_cluster_kernel<float>, (const void*)dense_cluster_kernel<double>,
         (const void*)solve_kernel<float, float>, (const void*)solve_kernel<float, double>,
         (const void*)solve_kernel<float, __half>, (const void*)solve_kernel<double, double>};
@@ -720,8 +739,9 @@ int preload_kernels() {
 }
 
 int refactor_occupancy(int prec, size_t smem, int block, int* occ, bool spread) {
-    if (prec == LUSP_FP64) return refactor_prepare<double>(smem, block, occ, spread);
-    return refactor_prepare<float>(smem, block, occ, spread);
+    const RefactorKind kind = spread ? kSpread : kLone;
+    if (prec == LUSP_FP64) return refactor_prepare<double>(smem, block, occ, kind);
+    return refactor_prepare<float>(smem, block, occ, kind);
 }
 
 int kernel_occupancy(int prec, int inner, size_t smem, int block, int* occ) {
@@ -761,8 +781,8 @@ static int launch_rung(const SysDev* sys, int nsys, int* q, const int* dyn, cons
     cudaError_t e;
     if (kev && cudaEventRecord(kev[0], st) != cudaSuccess) return cuda_fail(cudaGetLastError(), "timing event");
     if (what & LUSP_RUN_REFACTOR) {
-        const bool spread = r.rspread.group > 0;
-        int rc = refactor_prepare<VT>(r.rplan.bytes, r.rblock, nullptr, spread);
+        const RefactorKind kind = r.rspread.group > 0 ? kSpread : r.rcluster > 1 ? kCluster : kLone;
+        int rc = refactor_prepare<VT>(r.rplan.bytes, r.rblock, nullptr, kind);
         if (rc != LUSP_OK) return rc;
         if (r.rspread.group > 0) {
             // The systems' sync areas start at zero (claim counters, status
@@ -783,10 +803,10 @@ static int launch_rung(const SysDev* sys, int nsys, int* q, const int* dyn, cons
             attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            e = cudaLaunchKernelEx(&cfg, refactor_fn<VT>(r.rblock), sys, nsys, q, r.rplan, prm, dyn, list,
+            e = cudaLaunchKernelEx(&cfg, refactor_fn<VT>(r.rblock, kind), sys, nsys, q, r.rplan, prm, dyn, list,
                                    r.rspread);
         } else {
-            refactor_fn<VT>(r.rblock, spread)<<<r.rgrid, r.rblock, r.rplan.bytes, st>>>(sys, nsys, q, r.rplan, prm,
+            refactor_fn<VT>(r.rblock, kind)<<<r.rgrid, r.rblock, r.rplan.bytes, st>>>(sys, nsys, q, r.rplan, prm,
                                                                                      dyn, list, r.rspread);
             e = cudaGetLastError();
         }
@@ -889,7 +909,7 @@ int batch_launch(BatchObj* B, int what, cudaStream_t st, bool timed) {
 int tail_ld(const StaticPattern& S) { return (S.dtail + 31) & ~31; }
 
 static SysSizes host_sizes(const StaticPattern& S) {
-    return SysSizes{(size_t)S.n, (size_t)S.cap, S.lci.size(), S.uci.size(), (size_t)S.sell_ptr.back(),
+    return SysSizes{(size_t)S.n, (size_t)S.cap, (size_t)S.lp[S.k0], S.lci.size(), S.uci.size(), (size_t)S.sell_ptr.back(),
                     (size_t)S.dtail, (size_t)tail_ld(S)};
 }
 

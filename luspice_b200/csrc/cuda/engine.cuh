@@ -17,7 +17,8 @@ namespace lusp {
 // Device-resident static pattern (all pointers are device memory).
 struct PatternDev {
     int n, nnz_a, cap, max_col, nslices, sell_total;
-    int nnz_l, nnz_u;        // strict L and strict U entries
+    int nnz_l, nnz_u;        // strict L and strict U entries (by rows)
+    int nnz_lcol;            // strict L entries of the columns before the dense block
     int nfwd_levels, nbwd_levels;    // sweep steps (descriptors) of each sweep
     const int* cp;           // [n+1] merged column pointers
     const int* ri;           // [cap] row positions, ascending per column
@@ -41,10 +42,9 @@ struct PatternDev {
     const int* sell_perm;    // [32*nslices] row position or -1
     const int* rowat;        // [n] position -> original row
     const int* q;            // [n] position -> original column
-    const int2* dep_bc;           // [cap] for U slots: {first strict-L slot,
-                                  // strict-L length} of the dependency column
-    const unsigned short* rel;    // relative update slots (null: search rows)
-    const long long* rel_ptr;     // [n+1] column k's list in rel
+    const int* lp;           // [n+1] packed strict-L columns (SysDev::lcol)
+    const int4* seg;         // update segments (StaticPattern::seg; null: search rows)
+    const unsigned short* rel;    // ... and their relative slots
     // Dense trailing block: rows/columns [k0, n), dtail = n - k0 (0: none);
     // tail_ld: dtail rounded up to 32.
     int k0, dtail, tail_ld;
@@ -53,11 +53,11 @@ struct PatternDev {
     // refactor writes only these entries of the fp64 block; the dense kernel
     // reads every other entry as 0 in its first panel step.
     const unsigned* tail_mask;
-    // Column records of the refactorization, three 16-byte words per claim
+    // Column records of the refactorization, four 16-byte words per claim
     // index idx (column k = col_order[idx]): {k, cp[k], column length,
     // diagonal offset}, {first input entry a_ptr[k], a_ptr[k + 1],
     // dependencies before the dense block, bwd_pos[k]}, {rel_ptr[k] low and
-    // high words, a_diag[k], 0}.
+    // high words, a_diag[k], 0}, {seg_ptr[k], segments, lp[k], 0}.
     const int4* crec;
     const int* a_diag;       // [n] slot offset of A(q_k, q_k) in column k, or -1
     const int* bwd_pos;      // [n] row -> index in bwd_order
@@ -97,6 +97,7 @@ struct SysDev {
     const PatternDev* pat;
     const double* a_val;     // [nnz_a] input values, fp64
     void* lu;                // [cap] merged factor values (VT)
+    void* lcol;              // [nnz_lcol] packed strict L columns before the dense block (VT)
     void* lval;              // [nnz_l] strict L by rows (VT)
     void* uval;              // [nnz_u] strict U by rows (VT)
     void* udiag;             // [n] U(k,k) (VT)
@@ -129,7 +130,7 @@ struct SolveParams {
     double inner_rel;        // inner stop relative to the current residual
     double stag_ratio;       // residual must shrink by this factor per outer
     double pivot_tol;        // frozen-pivot acceptance threshold
-    int refactor_mode;       // 0 staged gathers (cp.async), 1 per-dependency loads
+    int refactor_mode;       // 0 segment updates, 1 per dependency with a row search
     double xtol;             // forward-error target of the refinement
     double shift;            // factor of A + shift * diag|A(i,i)| (0: A itself)
 };
@@ -145,11 +146,11 @@ __host__ __device__ inline size_t tail_index(int D, int r, int c) {
 
 // Sizes that fix one system's private device area.
 struct SysSizes {
-    size_t n, cap, nnz_l, nnz_u, sell, dtail, tail_ld;
+    size_t n, cap, nnz_lcol, nnz_l, nnz_u, sell, dtail, tail_ld;
 };
 
 __host__ __device__ inline SysSizes sizes_of(const PatternDev& P) {
-    return SysSizes{(size_t)P.n, (size_t)P.cap, (size_t)P.nnz_l, (size_t)P.nnz_u,
+    return SysSizes{(size_t)P.n, (size_t)P.cap, (size_t)P.nnz_lcol, (size_t)P.nnz_l, (size_t)P.nnz_u,
                     (size_t)P.sell_total, (size_t)P.dtail, (size_t)P.tail_ld};
 }
 
@@ -164,7 +165,7 @@ __host__ __device__ inline size_t tinv_bytes(const SysSizes& z, size_t vs) {
 }
 
 __host__ __device__ inline size_t sys_private_bytes(const SysSizes& z, size_t vs, int m) {
-    return al256(z.cap * vs + 64) + al256(z.nnz_l * vs + 64) + al256(z.nnz_u * vs + 64) + al256(z.n * vs) +
+    return al256(z.cap * vs + 64) + al256(z.nnz_lcol * vs + 64) + al256(z.nnz_l * vs + 64) + al256(z.nnz_u * vs + 64) + al256(z.n * vs) +
            al256(z.n * vs + 64) + al256(z.sell * 8) + al256(z.sell * 4) + al256((2 * (size_t)m + 8) * z.n * 8) +
            al256(z.dtail * z.tail_ld * vs) + al256(z.dtail * z.tail_ld * 8) + al256(z.sell * 2) +
            2 * al256(z.n * 8) + al256(tinv_bytes(z, vs));
@@ -178,6 +179,7 @@ __host__ __device__ inline char* sys_carve(SysDev& D, char* p, const SysSizes& z
     D.tailw = z.dtail > 0 ? (double*)p : nullptr;
     p += al256(z.dtail * z.tail_ld * 8);
     D.lu = p; p += al256(z.cap * vs + 64);
+    D.lcol = p; p += al256(z.nnz_lcol * vs + 64);
     D.lval = p; p += al256(z.nnz_l * vs + 64);
     D.uval = p; p += al256(z.nnz_u * vs + 64);
     D.udiag = p; p += al256(z.n * vs);
@@ -235,7 +237,6 @@ __host__ __device__ inline int sync_stride(int nmax) { return (kSyncReady + (nma
 struct SmemPlan {
     int nwords;              // ready-bit words (>= ceil(n_max/32))
     int wcap;                // per-warp refactor work slots
-    int scap;                // per-warp staged L entries (refactor gathers)
     int drows;               // dense trailing block: rows of a block column
     int dstg;                // ... and panel row groups in flight per warp (1 or 3)
     int sc_ent, sc_rows;     // sweep stage capacity (entries, rows; 0: no stages)

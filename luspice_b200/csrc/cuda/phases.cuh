@@ -636,17 +636,139 @@ __device__ void dense_phase(const SysDev& S, const SmemPlan& plan, char* smem_ba
 // Column k (one warp): x = A(:,k) scattered into the column's own slots
 // (duplicates summed in input order); for each U(:,k) row j ascending, once
 // column j is ready: x[s] -= L(i,j) * x[j] for the strict-L entries (i, j),
-// s = slot of row i in column k (precomputed relative slots; a binary search
-// in column k's rows when the pattern has none); U(:,k) = x[rows < k],
-// U(k,k) = x[k], L(:,k) = x[rows > k] / U(k,k).  The work vector is fp64;
-// multiply and subtract are separately rounded so the result is bitwise
-// reproducible on the host.  Values are stored as VT (fp32 for the mixed
-// path, fp64 for the plain path) in the merged column layout and in the
-// row-major copies used by the solves.
+// s = slot of row i in column k; U(:,k) = x[rows < k], U(k,k) = x[k], L(:,k) =
+// x[rows > k] / U(k,k).  The work vector is fp64; multiply and subtract are
+// separately rounded so the result is bitwise reproducible on the host.
+// Values are stored as VT (fp32 for the mixed path, fp64 for the plain path):
+// the strict-L part packed by columns (the later columns' gathers read it,
+// published first), in the merged layout, and in the row-major copies used by
+// the solves.
 //
-// Shared memory per warp: x[wcap] (fp64), a stage of scap L values (VT) and
-// scap + 16 relative slots.
+// The dependencies are applied in segments of consecutive columns of one
+// supernode (PatternDev::seg): a lane keeps its rows' x in registers over the
+// segment, the dependencies' own x are exchanged by shuffles, and only the
+// first dependency's row slots are read.  The n = 4050 grid has 3.5
+// dependencies per segment (23 k segments for 81 k dependencies of 41 rows),
+// the n = 40,000 circuit more, analog circuits 1.4.  Staging every
+// dependency's values and slots through shared memory took 250 instructions
+// per dependency and filled 57 % of the issue slots; what bounds the refactor
+// now is the chain of columns for few systems (a ready bit seen, the L values
+// from L2, the update, the division, the release fence: ~7 k cycles a level
+// on the grid against ~2 k for the bare round trips) and instructions per
+// column for many.  B200, refactor kernel: 50 grids 1.54 -> 0.99 ms (fp64
+// 1.59 -> 1.10), one grid 1.25 -> 0.81 ms, the n = 40,000 circuit 43.7 ->
+// 17.4 ms, 50 circuits n = 989 263 -> 218 us, 768 uneven circuits 4.80 ->
+// 4.13 ms.
+//
+// Shared memory per warp: the column's record, pivot minima, x[wcap] (fp64).
 // ---------------------------------------------------------------------------
+// One segment's update: dependencies [a, a + W) of a segment whose first
+// dependency has slot u0 and its cnt strict-L rows packed from lp0, their
+// slots at rel.  Row i of the update is dependency a itself (i = 0) or its
+// strict-L row i - 1; it takes part in the steps t < i (dependency a + t),
+// whose L value of row i > t is at pl[i], pl moving on by the column's length.
+// An L value of a finished column.  LONE: written by this CTA, so the SM's own
+// L1 has it; else past L1 (another SM may have written it).
+template <bool LONE, typename VT>
+__device__ __forceinline__ VT load_l(const VT* p) { return LONE ? *p : __ldcg(p); }
+
+template <typename VT, bool TWO, bool LONE>
+__device__ __forceinline__ void seg_rows(const VT* lcol, const unsigned short* rel, double* x, int u0, int a, int W,
+                                         int lp0, int cnt) {
+    const int lane = threadIdx.x & 31, R = cnt - a + 1;
+    const int la = lane < R ? lane : -1;      // steps t < la update row lane
+    const bool lb = TWO && lane + 32 < R;
+    const VT* pl = lcol + (lp0 + a * cnt - ((a * (a - 1)) >> 1) - 1 + lane);
+    int step = cnt - a - 1;
+    const int sa = la > 0 ? (int)__ldg(rel + a + lane - 1) : u0 + a;
+    const int sb = lb ? (int)__ldg(rel + a + lane + 31) : 0;
+    double xa = 0.0, xb = 0.0;
+    for (int t0 = 0; t0 < W; t0 += 4) {
+        VT va[4], vb[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (t0 + q >= W) break;
+            va[q] = t0 + q < la ? load_l<LONE>(pl) : VT(0);
+            if (TWO) vb[q] = lb ? load_l<LONE>(pl + 32) : VT(0);
+            pl += step;
+            step--;
+        }
+        if (t0 == 0) {
+            xa = x[sa];
+            if (TWO) xb = x[sb];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (t0 + q >= W) break;
+            const double xj = __shfl_sync(0xffffffffu, xa, t0 + q);
+            if (xj != 0.0) {
+                if (t0 + q < la) xa = __dsub_rn(xa, __dmul_rn((double)va[q], xj));
+                if (lb) xb = __dsub_rn(xb, __dmul_rn((double)vb[q], xj));
+            }
+        }
+    }
+    if (la > 0) x[sa] = xa;
+    if (lb) x[sb] = xb;
+    if (!TWO) return;
+    // Rows from 64 on, 64 at a time, with the dependencies' final x.
+    for (int i0 = 64; i0 < R; i0 += 64) {
+        const bool pa = i0 + lane < R, pb = i0 + lane + 32 < R;
+        const VT* ph = lcol + (lp0 + a * cnt - ((a * (a - 1)) >> 1) - 1 + lane + i0);
+        int hs = cnt - a - 1;
+        const int ra = pa ? (int)__ldg(rel + a + i0 + lane - 1) : 0, rb = pb ? (int)__ldg(rel + a + i0 + lane + 31) : 0;
+        double ya = x[ra], yb = x[rb];
+        for (int t0 = 0; t0 < W; t0 += 4) {
+            VT va[4], vb[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (t0 + q >= W) break;
+                va[q] = pa ? load_l<LONE>(ph) : VT(0);
+                vb[q] = pb ? load_l<LONE>(ph + 32) : VT(0);
+                ph += hs;
+                hs--;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (t0 + q >= W) break;
+                const double xj = __shfl_sync(0xffffffffu, xa, t0 + q);
+                if (xj != 0.0) {
+                    if (pa) ya = __dsub_rn(ya, __dmul_rn((double)va[q], xj));
+                    if (pb) yb = __dsub_rn(yb, __dmul_rn((double)vb[q], xj));
+                }
+            }
+        }
+        if (pa) x[ra] = ya;
+        if (pb) x[rb] = yb;
+    }
+}
+
+template <typename VT, bool LONE>
+__device__ __forceinline__ void seg_update(const VT* lcol, const unsigned short* rel, double* x, int u0, int a, int W,
+                                           int lp0, int cnt) {
+    if (W == 1) {
+        // One dependency: a multiply-subtract per row, two rows per lane in
+        // flight.
+        const int lane = threadIdx.x & 31, m = cnt - a;
+        const VT* src = lcol + (lp0 + a * cnt - ((a * (a - 1)) >> 1));
+        const double xj = x[u0 + a];
+        if (xj != 0.0) {
+            for (int e = lane; e < m; e += 64) {
+                const bool two = e + 32 < m;
+                const int s0 = (int)__ldg(rel + a + e), s1 = two ? (int)__ldg(rel + a + e + 32) : s0;
+                const VT l0 = load_l<LONE>(src + e), l1 = two ? load_l<LONE>(src + e + 32) : VT(0);
+                const double x0 = x[s0], x1 = x[s1];
+                x[s0] = __dsub_rn(x0, __dmul_rn((double)l0, xj));
+                if (two) x[s1] = __dsub_rn(x1, __dmul_rn((double)l1, xj));
+            }
+        }
+    } else if (cnt - a < 32) {
+        seg_rows<VT, false, LONE>(lcol, rel, x, u0, a, W, lp0, cnt);
+    } else {
+        seg_rows<VT, true, LONE>(lcol, rel, x, u0, a, W, lp0, cnt);
+    }
+    __syncwarp();
+}
+
 // Spread mode: the pivot statistics and cycle counters of one CTA merged
 // into the system's sync area; the last CTA to finish writes the system's
 // statistics (pivot minima through the bit patterns of non-negative doubles:
@@ -708,32 +830,57 @@ __device__ __forceinline__ long long phase_clock() {
     else return 0;
 }
 
+// A CTA's copy of its system's descriptors in shared memory: the column loop
+// reads each pointer where it uses it (30 cycles) instead of holding some
+// sixty registers of them or fetching them from global memory.
+struct RefactorCtx {
+    SysDev sys;
+    PatternDev pat;
+};
+
+// Pause between two looks at the ready bits of a column's dependencies.
+constexpr unsigned kPollSleep = 32;
+
+// Bytes of a warp's column record and pivot minima, before its work vector.
+constexpr int kWarpHead = 80;
+
+// All threads; ends with a CTA barrier.
+__device__ __forceinline__ void load_ctx(RefactorCtx& cx, const SysDev* sys) {
+    static_assert(sizeof(SysDev) % 4 == 0 && sizeof(PatternDev) % 4 == 0, "copied as words");
+    const int* pat = (const int*)sys->pat;
+    for (int t = threadIdx.x; t < (int)(sizeof(SysDev) / 4); t += blockDim.x) ((int*)&cx.sys)[t] = ((const int*)sys)[t];
+    for (int t = threadIdx.x; t < (int)(sizeof(PatternDev) / 4); t += blockDim.x) ((int*)&cx.pat)[t] = pat[t];
+    __syncthreads();
+}
+
 // SPREAD: the system's columns are shared by `group` CTAs anywhere on the
 // GPU (CTA `member` of them) through the sync area in global memory; else
 // by the CTAs of this thread-block cluster through rank 0's shared memory.
-template <typename VT, bool SPREAD = false>
-__device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem_base,
+// LONE: by this CTA alone, through its own shared memory.
+template <typename VT, bool SPREAD = false, bool LONE = false>
+__device__ void refactor_phase(const RefactorCtx& cx, const SmemPlan& plan, char* smem_base,
                                const SolveParams& prm, unsigned* sync = nullptr, int member = 0,
                                int group = 1) {
-    const PatternDev& P = *S.pat;
+    const SysDev& S = cx.sys;
+    const PatternDev& P = cx.pat;
     const int n = P.n;
     Smem sm(smem_base, plan);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const size_t per_warp = (size_t)plan.wcap * 8 + (size_t)plan.scap * sizeof(VT) + ((size_t)plan.scap + 16) * 2;
-    char* wbase = sm.uni + (size_t)warp * per_warp;
-    double* wx = (double*)wbase;
-    VT* sval = (VT*)(wbase + (size_t)plan.wcap * 8);
-    unsigned short* srel = (unsigned short*)(wbase + (size_t)plan.wcap * 8 + (size_t)plan.scap * sizeof(VT));
-    const bool have_rel = P.rel != nullptr && prm.refactor_mode == 0;
+    // This warp's column record (16 ints), pivot minima and work vector.
+    int* rec = (int*)(sm.uni + (size_t)warp * ((size_t)plan.wcap * 8 + kWarpHead));
+    double* pmin = (double*)(rec + 16);
+    double* wx = pmin + 2;
+    if (lane == 0) pmin[0] = pmin[1] = INFINITY;
+    const bool have_seg = P.seg != nullptr && prm.refactor_mode == 0;
     // The CTAs of a thread-block cluster share one system: the claim
     // counter, status, singular column, abort flag and ready bits live in
     // rank 0's shared memory (distributed shared memory for the others).
     namespace cgr = cooperative_groups;
     cgr::cluster_group cl = cgr::this_cluster();
-    const unsigned crank = SPREAD ? (unsigned)member : cl.block_rank();
-    const unsigned csize = SPREAD ? (unsigned)group : cl.num_blocks();
-    unsigned* ready = SPREAD ? sync + kSyncReady : cl.map_shared_rank(sm.ready, 0);
-    int* ctl = SPREAD ? (int*)sync : cl.map_shared_rank(sm.ctl, 0);
+    const unsigned crank = SPREAD ? (unsigned)member : LONE ? 0u : cl.block_rank();
+    const unsigned csize = SPREAD ? (unsigned)group : LONE ? 1u : cl.num_blocks();
+    unsigned* ready = SPREAD ? sync + kSyncReady : LONE ? sm.ready : cl.map_shared_rank(sm.ready, 0);
+    int* ctl = SPREAD ? (int*)sync : LONE ? sm.ctl : cl.map_shared_rank(sm.ctl, 0);
 
     if (!SPREAD && crank == 0) {
         for (int t = threadIdx.x; t < (n + 31) / 32; t += blockDim.x) sm.ready[t] = 0u;
@@ -744,17 +891,9 @@ __device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem
             sm.ctl[3] = 0;
         }
     }
-    // The system's dense trailing block: the tail columns scatter their
-    // pattern's entries into it (the dense kernel reads the others as 0).
-    double* W = P.dtail > 0 ? S.tailw : nullptr;
-
-    VT* lu = (VT*)S.lu;
-    VT* lval = (VT*)S.lval;
-    VT* uval = (VT*)S.uval;
-    VT* udiag = (VT*)S.udiag;
-    double minpiv = INFINITY, minratio = INFINITY, maxu = 0.0;
+    double maxu = 0.0;
     int bad = 0;
-    long long c_wait = 0, c_gather = 0, c_update = 0;
+    long long c_wait = 0, c_update = 0;
     const long long t_begin = clock64();
     if (!SPREAD) {
         if (crank == 0 && threadIdx.x == 0) {
@@ -762,28 +901,27 @@ __device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem
             S.stats->cyc_gather = 0;
             S.stats->cyc_update = 0;
         }
-        cl.sync();
+        if (LONE) __syncthreads();
+        else cl.sync();
     }
 
     while (true) {
         const int idx = warp_claim(&ctl[0]);
         if (idx >= n) break;
-        // The column's record (one broadcast load of three 16-byte words),
-        // then, all in flight together: this lane's first input entry, its
-        // first dependency, the destination of its first slot, and the input
-        // value.  The later entries (columns longer than a warp) load as
-        // they are reached.
-        const int4 ra = P.crec[3 * idx], rb = P.crec[3 * idx + 1], rc = P.crec[3 * idx + 2];
-        const int k = ra.x, c0 = ra.y, len = ra.z, d = ra.w;
-        const int a0 = rb.x, a1 = rb.y, dsp = rb.z, bpos = rb.w;
-        const int* rows = P.ri + c0;
+        // The column's record, four 16-byte words into shared memory, then,
+        // all in flight together: this lane's first input entry, its first
+        // segment, the destination of its first slot, and the input value.
+        // The later entries (columns longer than a warp) load as they are
+        // reached.
+        if (lane < 4) *(int4*)(rec + 4 * lane) = __ldg(P.crec + 4 * idx + lane);
+        __syncwarp();
+        const int len = rec[2], a0 = rec[4], a1 = rec[5], nseg = have_seg ? rec[13] : 0;
         const int ta = a0 + lane;
         const int adst = ta < a1 ? P.a_dst[ta] : -1;
         const int asrc = ta < a1 ? P.a_src[ta] : -1;
         const int aprev = (ta < a1 && ta > a0) ? P.a_dst[ta - 1] : -1;
-        const int jj0 = lane < dsp ? rows[lane] : 0;
-        const int2 bc0 = lane < dsp ? P.dep_bc[c0 + lane] : make_int2(0, 0);
-        const int sdst0 = lane < len ? P.slot_dst[c0 + lane] : -1;
+        int4 sg = lane < nseg ? __ldg(P.seg + rec[12] + lane) : make_int4(0, 0, 0, 0);
+        const int sdst0 = lane < len ? P.slot_dst[rec[1] + lane] : -1;
         const double av0 = asrc >= 0 ? S.a_val[asrc] : 0.0;
         double* x;
         if (len <= plan.wcap) {
@@ -793,17 +931,14 @@ __device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem
         } else {
             bad |= ST_CAPACITY;
             __syncwarp();
-            if (lane == 0) set_ready(ready, k);
+            if (lane == 0) set_ready(ready, rec[0]);
             continue;
         }
-        // A column of the dense trailing block applies only its dependencies
-        // before k0 here (they come first: rows ascending; dsp of them).
-        const bool tailcol = k >= P.k0;
         for (int t = lane; t < len; t += 32) x[t] = 0.0;
         __syncwarp();
         // The factor of A + shift diag|A(i,i)|: the input's diagonal entry
         // (duplicates summed first) gains shift times its magnitude.
-        const int adg = prm.shift != 0.0 ? rc.z : -1;
+        const int adg = prm.shift != 0.0 ? rec[10] : -1;
         if (ta < a1 && (ta == a0 || aprev != adst)) {
             double s = av0;
             for (int u = ta + 1; u < a1 && P.a_dst[u] == adst; u++) s = __dadd_rn(s, S.a_val[P.a_src[u]]);
@@ -822,186 +957,125 @@ __device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem
         }
         __syncwarp();
         long long tc = phase_clock();
-        // Apply the dependency columns in ascending order.  Each round takes
-        // the next run of dependencies that are already complete (blocking
-        // only when the very next one is not, so the older dependencies of a
-        // column overlap with the computation of its most recent ones), up to
-        // plan.scap gathered entries; their L values and relative slots are
-        // copied to shared memory with all copies in flight together, then
-        // applied.
-        // rel index of dependency u0
-        long long roff = have_rel ? (long long)(((unsigned long long)(unsigned)rc.y << 32) | (unsigned)rc.x) : 0;
-        // Dependency metadata of the round starting at pf_u0, loaded while
-        // the previous round's copies and updates ran.
-        int pf_u0 = 0, pf_jj = jj0;
-        int2 pf_bc = bc0;
-        for (int u0 = 0; u0 < dsp;) {
-            const int u = u0 + lane;
-            int beg = 0, cnt = 0;
-            bool rdy = true;
-            if (u < dsp) {
-                const bool pre = u0 == pf_u0;
-                const int jj = pre ? pf_jj : rows[u];
-                const int2 bc = pre ? pf_bc : P.dep_bc[c0 + u];
-                beg = bc.x;
-                cnt = bc.y;
-                rdy = is_ready(ready, jj);
-            }
-            // Acquire (spread mode): each lane orders what follows after its
-            // own ready-bit read; the warp's ballot then orders the other
-            // lanes' reads of that dependency's values after it.
-            if (SPREAD) spread_acquire();
-            int nready = __ffs(~__ballot_sync(0xffffffffu, rdy)) - 1;
-            if (nready < 0) nready = 32;
-            if (nready == 0) {
-                // Wait for the next dependency, then re-scan: others may
-                // have completed meanwhile and join the same round.
-                const bool ok = __all_sync(0xffffffffu, wait_ready(ready, rows[u0], &ctl[3]));
-                if (ok) continue;
-                bad |= ST_WAIT_TIMEOUT;
-                nready = 1;
-            }
-            // Acquire (cluster): the dependency columns' values (written by
-            // any CTA of the cluster) are read after their ready bits.
-            if (!SPREAD) share_fence(csize);
-            {
-                const long long t2 = phase_clock();
-                c_wait += t2 - tc;
-                tc = t2;
-            }
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            const int excl = incl - cnt;
-            // Value stage layout: each dependency's run starts at the 16-byte
-            // boundary at or below its first value (copied in whole 16-byte
-            // pieces that bypass L1, so values written by another SM are never
-            // read from a stale L1 line).
-            constexpr int VPK = 16 / (int)sizeof(VT);
-            const int vsh = beg & (VPK - 1);
-            const int vlen = u < dsp ? ((vsh + cnt + VPK - 1) / VPK) * VPK : 0;
-            int vincl = vlen;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, vincl, o);
-                if (lane >= o) vincl += v;
-            }
-            const int vexcl = vincl - vlen;
-            int nfit = have_rel ? __popc(__ballot_sync(0xffffffffu, u < dsp && incl <= plan.scap &&
-                                                                        vincl <= plan.scap))
-                                : 0;
-            nfit = min(nfit, nready);
-            if (nfit == 0) {
-                // One dependency applied straight from global memory (longer
-                // than the stage, or no relative slots).
-                const double xj = x[u0];
-                const int p0 = __shfl_sync(0xffffffffu, beg, 0);
-                const int c = __shfl_sync(0xffffffffu, cnt, 0);
-                if (xj != 0.0) {
-                    for (int e = lane; e < c; e += 32) {
-                        const double l = (double)__ldcg(lu + p0 + e);
-                        const int s = have_rel ? (int)P.rel[roff + e]
-                                               : find_slot(rows, u0 + 1, len, P.ri[p0 + e]);
-                        if (s >= 0) x[s] = __dsub_rn(x[s], __dmul_rn(l, xj));
-                        else bad |= ST_CAPACITY;
-                    }
+        // Apply the dependency columns in ascending order, 32 segments at a
+        // time: each round takes the segments whose dependencies are all
+        // complete, up to the first that is not, then the complete first part
+        // of that one; it blocks only when nothing could be applied.
+        const unsigned short* rel = P.rel + *(const long long*)(rec + 8);
+        const VT* lcol = (const VT*)S.lcol;
+        for (int s0 = 0; s0 < nseg; s0 += 32) {
+            if (s0 > 0) sg = s0 + lane < nseg ? __ldg(P.seg + rec[12] + s0 + lane) : make_int4(0, 0, 0, 0);
+            const int ns = min(32, nseg - s0);
+            const int jj = sg.x, w = sg.y >> 16;
+            int c = 0, off = 0;     // next segment of the window, its dependencies already applied
+            long long spins = 0;    // looks since the last one that found work
+            while (c < ns) {
+                int r = 0;
+                if (lane >= c && lane < ns) {
+                    // Ready bits of columns jj .. jj + w - 1 (w <= 32).
+                    const int sh = jj & 31;
+                    const volatile unsigned* word = ready + (jj >> 5);
+                    unsigned bits = word[0] >> sh;
+                    if (sh + w > 32) bits |= word[1] << (32 - sh);
+                    r = min(w, bits == 0xffffffffu ? 32 : __ffs(~bits) - 1);
                 }
-                __syncwarp();
-                roff += c;
-                u0 += 1;
-                continue;
-            }
-            // Stage: relative slots of the round (one contiguous run of rel,
-            // copied in aligned 16-byte pieces) and each dependency's values.
-            const int tot = __shfl_sync(0xffffffffu, incl, nfit - 1);
-            const long long g0 = roff & ~7LL;
-            const int sh = (int)(roff - g0);
-            const int pieces = (sh + tot + 7) >> 3;
-            for (int e = lane; e < pieces; e += 32) cp_async_16(srel + 8 * e, P.rel + g0 + 8 * e);
-            for (int t = 0; t < nfit; t++) {
-                const int a_t = __shfl_sync(0xffffffffu, beg - vsh, t);
-                const int p_t = __shfl_sync(0xffffffffu, vlen, t) / VPK;
-                const int o_t = __shfl_sync(0xffffffffu, vexcl, t);
-                for (int e = lane; e < p_t; e += 32) cp_async_16(sval + o_t + e * VPK, lu + a_t + e * VPK);
-            }
-            // The next round's metadata, in flight with the copies.
-            pf_u0 = u0 + nfit;
-            if (pf_u0 + lane < dsp) {
-                pf_jj = __ldg(rows + pf_u0 + lane);
-                pf_bc = __ldg(P.dep_bc + c0 + pf_u0 + lane);
-            }
-            cp_async_wait_all();
-            __syncwarp();
-            {
-                const long long t2 = phase_clock();
-                c_gather += t2 - tc;
-                tc = t2;
-            }
-            for (int t = 0; t < nfit; t++) {
-                const int c_t = __shfl_sync(0xffffffffu, cnt, t);
-                const int o_t = __shfl_sync(0xffffffffu, excl, t);
-                const int vo_t = __shfl_sync(0xffffffffu, vexcl + vsh, t);
-                const double xj = x[u0 + t];
-                if (xj != 0.0 && c_t <= 32) {
-                    // A short dependency column: one entry per lane.
-                    if (lane < c_t) {
-                        const int s = (int)srel[sh + o_t + lane];
-                        const double l = ValTraits<VT>::load(sval + vo_t + lane);
-                        x[s] = __dsub_rn(x[s], __dmul_rn(l, xj));
-                    }
-                } else if (xj != 0.0 && c_t <= 64) {
-                    // Two entries per lane, both loaded before either store
-                    // (rows of one dependency are distinct).
-                    const bool h = lane + 32 < c_t;
-                    const int s0 = (int)srel[sh + o_t + lane];
-                    const int s1 = h ? (int)srel[sh + o_t + lane + 32] : s0;
-                    const double l0 = ValTraits<VT>::load(sval + vo_t + lane);
-                    const double l1 = h ? ValTraits<VT>::load(sval + vo_t + lane + 32) : 0.0;
-                    const double x0 = x[s0], x1 = x[s1];
-                    x[s0] = __dsub_rn(x0, __dmul_rn(l0, xj));
-                    if (h) x[s1] = __dsub_rn(x1, __dmul_rn(l1, xj));
-                } else if (xj != 0.0) {
-                    // Rows of one dependency are distinct: four entries per
-                    // lane are loaded before any is written back.
-                    for (int e = lane; e < c_t; e += 128) {
-                        int s[4];
-                        double l[4], xv[4];
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const int ee = e + 32 * q;
-                            s[q] = ee < c_t ? (int)srel[sh + o_t + ee] : -1;
-                            l[q] = ee < c_t ? ValTraits<VT>::load(sval + vo_t + ee) : 0.0;
+                // Acquire: each lane orders what follows after its own reads
+                // of ready bits; the warp's ballot then orders the other
+                // lanes' reads of those columns' values after them.
+                if (SPREAD) spread_acquire();
+                const unsigned full = __ballot_sync(0xffffffffu, lane >= c && lane < ns && r >= w) >> c;
+                int run = full == 0xffffffffu ? 32 : __ffs(~full) - 1;
+                int part = 0;        // applied part of the segment after the run
+                bool late = false;
+                if (c + run < ns) {
+                    part = __shfl_sync(0xffffffffu, r, c + run);
+                    if (run == 0 && part <= off) {
+                        // Nothing to apply yet.  Spread mode: look again (the
+                        // look is the poll: a wait for one bit and then a look
+                        // would read the bits twice, 340 cycles each).  Else
+                        // the bits are near: wait for the next dependency.
+                        if (!SPREAD) {
+                            const int jn = __shfl_sync(0xffffffffu, jj, c) + off;
+                            if (__all_sync(0xffffffffu, wait_ready(ready, jn, &ctl[3]))) continue;
+                        } else if (++spins <= kSpinLimit && ((spins & 31) || !*(const volatile int*)&ctl[3])) {
+                            __nanosleep(kPollSleep);
+                            continue;
                         }
-#pragma unroll
-                        for (int q = 0; q < 4; q++) xv[q] = s[q] >= 0 ? x[s[q]] : 0.0;
-#pragma unroll
-                        for (int q = 0; q < 4; q++)
-                            if (s[q] >= 0) x[s[q]] = __dsub_rn(xv[q], __dmul_rn(l[q], xj));
+                        if (SPREAD && spins > kSpinLimit) atomicExch(&ctl[3], 1);
+                        spins = kSpinLimit;
+                        bad |= ST_WAIT_TIMEOUT;
+                        part = off + 1;
+                        late = true;
                     }
                 }
-                __syncwarp();
+                if (!late) spins = 0;
+                // Acquire (cluster): the dependency columns' values (written
+                // by any CTA of the cluster) are read after their ready bits.
+                if (!SPREAD) share_fence(csize);
+                {
+                    const long long t2 = phase_clock();
+                    c_wait += t2 - tc;
+                    tc = t2;
+                }
+                const int end = c + run + ((part > 0 && (run > 0 || part > off)) ? 1 : 0);
+                for (int s = c; s < end; s++) {
+                    const int y = __shfl_sync(0xffffffffu, sg.y, s), lp0 = __shfl_sync(0xffffffffu, sg.z, s);
+                    const int cnt = __shfl_sync(0xffffffffu, sg.w, s);
+                    const int a = s == c ? off : 0;
+                    seg_update<VT, LONE>(lcol, rel, x, y & 0xffff, a, (s < c + run ? y >> 16 : part) - a, lp0, cnt);
+                    if (s < c + run) rel += cnt;
+                }
+                if (run > 0) off = 0;
+                if (part > off) off = part;
+                c += run;
+                if (late && off >= __shfl_sync(0xffffffffu, w, c)) {
+                    rel += __shfl_sync(0xffffffffu, sg.w, c);
+                    off = 0;
+                    c++;
+                }
+                {
+                    const long long t2 = phase_clock();
+                    c_update += t2 - tc;
+                    tc = t2;
+                }
             }
-            {
-                const long long t2 = phase_clock();
-                c_update += t2 - tc;
-                tc = t2;
-            }
-            roff += tot;
-            u0 += nfit;
         }
-        if (tailcol) {
-            // U rows before k0 are final; the rest goes to the dense block
-            // (destinations of four slots per lane loaded first).
+        // Without segments: one dependency at a time, its rows searched.
+        for (int u = 0; !have_seg && u < rec[6]; u++) {
+            const int* rows = P.ri + rec[1];
+            const int j = rows[u];
+            if (!__all_sync(0xffffffffu, wait_ready(ready, j, &ctl[3]))) bad |= ST_WAIT_TIMEOUT;
+            if (SPREAD) spread_acquire();
+            else share_fence(csize);
+            const double xj = x[u];
+            const int p0 = P.lp[j], cn = P.lp[j + 1] - p0;
+            if (xj != 0.0) {
+                for (int e = lane; e < cn; e += 32) {
+                    const double l = (double)__ldcg(lcol + p0 + e);
+                    const int s = find_slot(rows, u + 1, len, P.ri[P.dg[j] + 1 + e]);
+                    if (s >= 0) x[s] = __dsub_rn(x[s], __dmul_rn(l, xj));
+                    else bad |= ST_CAPACITY;
+                }
+            }
+            __syncwarp();
+        }
+        const int k = rec[0], c0 = rec[1], d = rec[3];
+        // A column of the dense trailing block applies only its dependencies
+        // before k0 here (they come first: rows ascending; dsp of them).
+        if (k >= P.k0) {
+            // U rows before k0 are final; the rest goes to the dense block,
+            // its pattern's entries (the dense kernel reads the others as 0;
+            // destinations of four slots per lane loaded first).
+            const int dsp = rec[6], k0 = P.k0, D = P.dtail;
+            double* W = S.tailw;
+            VT* uval = (VT*)S.uval;
             for (int t0 = lane; t0 < len; t0 += 128) {
                 int dst[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const int t = t0 + 32 * q;
                     dst[q] = t >= len ? 0 : t < dsp ? (t < 32 ? sdst0 : __ldg(P.slot_dst + c0 + t))
-                                                    : __ldg(rows + t);
+                                                    : __ldg(P.ri + c0 + t);
                 }
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
@@ -1012,17 +1086,33 @@ __device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem
                         maxu = fmax(maxu, fabs(v));
                         uval[dst[q]] = ValTraits<VT>::to(v);
                     } else {
-                        W[tail_index(P.dtail, dst[q] - P.k0, k - P.k0)] = v;
+                        W[tail_index(D, dst[q] - k0, k - k0)] = v;
                     }
                 }
             }
             __syncwarp();
             continue;
         }
-        const double piv = x[d];
+        const double piv = x[d], rpiv = __drcp_rn(piv);
+        // The multipliers, published before anything else of the column.
+        // amax: the largest |x| below the pivot whose multiplier is at least
+        // 1 in magnitude (the others are below the pivot, so they do not
+        // count for its ratio).
         double amax = 0.0;
-        for (int t = d + 1 + lane; t < len; t += 32) amax = fmax(amax, fabs(x[t]));
-        amax = warp_max(amax);
+        VT* lk = (VT*)S.lcol + rec[14] - d - 1;
+#pragma unroll 4
+        for (int t = d + 1 + lane; t < len; t += 32) {
+            const double v = x[t];
+            const VT l = ValTraits<VT>::to(div_by<false>(v, piv, rpiv));
+            lk[t] = l;
+            x[t] = (double)l;
+            if (fabs((double)l) >= 1.0) amax = fmax(amax, fabs(v));
+        }
+        // Release: the column's values before its ready bit.
+        share_release_t<SPREAD>(csize);
+        __syncwarp();
+        if (lane == 0) set_ready(ready, k);
+        if (__any_sync(0xffffffffu, amax > 0.0)) amax = warp_max(amax);
         const double ap = fabs(piv);
         if (!(ap > 0.0) || !isfinite(piv)) {
             bad |= ST_SINGULAR;
@@ -1033,16 +1123,20 @@ __device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem
                 else atomicMin(&ctl[2], k);
             }
         }
-        minpiv = fmin(minpiv, ap);
         const double ratio = amax > ap ? ap / amax : 1.0;
-        minratio = fmin(minratio, ratio);
+        if (lane == 0) {
+            pmin[0] = fmin(pmin[0], ap);
+            pmin[1] = fmin(pmin[1], ratio);
+        }
         if (ratio < prm.pivot_tol) bad |= ST_PIVOT_WEAK;
-        const double rpiv = __drcp_rn(piv);
         // Each value is stored once where the solves read it (U rows, the
         // diagonal, L rows); the strict-L part also goes to the merged
-        // columns, which the later columns' gathers read.  The destinations
-        // of four slots per lane are loaded before any of their stores (the
-        // loads could not move above the stores of an earlier slot).
+        // columns.  The destinations of four slots per lane are loaded before
+        // any of their stores (the loads could not move above the stores of
+        // an earlier slot).
+        VT* lu = (VT*)S.lu + c0;
+        VT* lval = (VT*)S.lval;
+        VT* uval = (VT*)S.uval;
         for (int t0 = lane; t0 < len; t0 += 128) {
             int dst[4];
 #pragma unroll
@@ -1054,39 +1148,41 @@ __device__ void refactor_phase(const SysDev& S, const SmemPlan& plan, char* smem
             for (int q = 0; q < 4; q++) {
                 const int t = t0 + 32 * q;
                 if (t >= len) break;
-                double v = x[t];
-                if (t > d) v = div_by(v, piv, rpiv);
-                else maxu = fmax(maxu, fabs(v));
+                const double v = x[t];
                 const VT sv = ValTraits<VT>::to(v);
+                if (t <= d) maxu = fmax(maxu, fabs(v));
                 if (t < d) uval[dst[q]] = sv;
                 else if (t == d) {
-                    udiag[k] = sv;
-                    ((VT*)S.udiag_bwd)[bpos] = ValTraits<VT>::to(rpiv);
+                    ((VT*)S.udiag)[k] = sv;
+                    ((VT*)S.udiag_bwd)[rec[7]] = ValTraits<VT>::to(rpiv);
                 } else {
-                    lu[c0 + t] = sv;
+                    lu[t] = sv;
                     lval[dst[q]] = sv;
                 }
             }
         }
-        // Release: the column's values before its ready bit.
-        share_release_t<SPREAD>(csize);
         __syncwarp();
-        if (lane == 0) set_ready(ready, k);
     }
 
+    __syncwarp();
+    const double minpiv = pmin[0], minratio = pmin[1];
     if (SPREAD) {
-        spread_finish(S, sync, group, sm, minpiv, minratio, maxu, bad, c_wait, c_gather, c_update, t_begin);
+        spread_finish(S, sync, group, sm, minpiv, minratio, maxu, bad, c_wait, 0, c_update, t_begin);
         return;
     }
     if (lane == 0) {
         atomicAdd((unsigned long long*)&S.stats->cyc_wait, (unsigned long long)c_wait);
-        atomicAdd((unsigned long long*)&S.stats->cyc_gather, (unsigned long long)c_gather);
         atomicAdd((unsigned long long*)&S.stats->cyc_update, (unsigned long long)c_update);
     }
     if (threadIdx.x == 0) S.stats->cyc_refactor = clock64() - t_begin;
     // Statistics: rank 0 writes, the others merge, one after another; the
     // last cluster barrier also keeps rank 0's shared state alive until every
     // CTA of the cluster is done with it.
+    if (LONE) {
+        __syncthreads();
+        cta_store_pivot_stats(S.stats, sm, minpiv, minratio, maxu, bad, true, ctl);
+        return;
+    }
     cl.sync();
     for (unsigned r = 0; r < csize; r++) {
         if (crank == r) cta_store_pivot_stats(S.stats, sm, minpiv, minratio, maxu, bad, r == 0, ctl);

@@ -89,16 +89,25 @@ struct StaticPattern {
     long flops = 0;                 // multiply-adds of one refactorization
     long gathered = 0;              // sum over deps of |L(:,j)| (entries)
 
-    // Relative slots of the refactorization updates: for column k, for each
-    // dependency j (rows of U(:,k) ascending), for each strict-L entry of
-    // column j in storage order, the slot offset inside column k that the
-    // entry updates.  Column k's list is rel[rel_ptr[k] .. rel_ptr[k+1]).
-    // Empty when a column is longer than 65535 slots.
+    // Strict L by columns, packed (the refactorization's gather source):
+    // column j is [lp[j], lp[j + 1]), rows ascending.
+    std::vector<int> lp;
+
+    // Update segments of the refactorization.  Consecutive columns j, j + 1
+    // form a supernode when L(:,j) below the diagonal is row j + 1 and then
+    // the rows of L(:,j + 1).  A dependency of column k inside a supernode
+    // brings all its later columns along (fill), in consecutive slots, so the
+    // dependencies of column k before the dense block fall into segments of
+    // consecutive columns of one supernode (at most kMaxSegment): segments
+    // [seg_ptr[k], seg_ptr[k + 1]), four ints each: first dependency column,
+    // its slot | length << 16, lp of that column, its strict-L length.
+    // rel[rel_ptr[k] ...): per segment, the slots inside column k of the
+    // strict-L rows of its first dependency (a later one's are the same
+    // list without its first entries).  Empty when a column is longer than
+    // 65535 slots.
+    std::vector<int> seg_ptr, seg;
     std::vector<uint16_t> rel;
     std::vector<long long> rel_ptr;
-    // For each U slot p of column k (row j): {dg[j] + 1, cp[j+1] - dg[j] - 1},
-    // the strict-L part of the dependency column (2 ints per slot, all slots).
-    std::vector<int> dep_bc;
 
     // Dense trailing block: rows and columns [k0, n) are refactored and
     // solved as one dense D x D block (D = dtail = n - k0; 0 = none).  The
@@ -107,6 +116,9 @@ struct StaticPattern {
     // the tail rows' entries in the columns before k0.
     int k0 = 0, dtail = 0;
 };
+
+// Longest update segment (a warp keeps a segment's values in its lanes).
+constexpr int kMaxSegment = 32;
 
 // Largest dense trailing block.
 constexpr int kMaxDenseTail = 768;

@@ -319,50 +319,62 @@ void build_static_pattern(int n, const int* Ap, const int* Ai, const int* q,
         S.gathered = ga;
     }
 
-    // Dependency metadata per U slot.
-    S.dep_bc.assign((size_t)S.cap * 2, 0);
-    for (int k = 0; k < n; k++)
-        for (int p = S.cp[k]; p < S.dg[k]; p++) {
-            const int j = S.ri[p];
-            S.dep_bc[(size_t)p * 2] = S.dg[j] + 1;
-            S.dep_bc[(size_t)p * 2 + 1] = S.cp[j + 1] - S.dg[j] - 1;
-        }
-
-    // Relative update slots (16 bit), built through a row -> slot table of
-    // the current column.
-    S.rel.clear();
-    S.rel_ptr.clear();
-    if (S.max_col <= 65535) {
-        S.rel.reserve((size_t)S.gathered);
-        S.rel_ptr.assign(n + 1, 0);
-        std::vector<int> at(n, -1);
-        bool closed = true;
-        for (int k = 0; k < n && closed; k++) {
-            S.rel_ptr[k] = (long long)S.rel.size();
-            for (int p = S.cp[k]; p < S.cp[k + 1]; p++) at[S.ri[p]] = p - S.cp[k];
-            for (int p = S.cp[k]; p < S.dg[k]; p++) {
-                const int j = S.ri[p];
-                for (int t = S.dg[j] + 1; t < S.cp[j + 1]; t++) {
-                    const int s = at[S.ri[t]];
-                    if (s < 0) closed = false;   // pattern not closed under the updates
-                    S.rel.push_back((uint16_t)s);
-                }
-            }
-            for (int p = S.cp[k]; p < S.cp[k + 1]; p++) at[S.ri[p]] = -1;
-        }
-        S.rel_ptr[n] = (long long)S.rel.size();
-        if (!closed) {
-            S.rel.clear();
-            S.rel_ptr.clear();
-        }
-    }
-
     // Dense trailing block.
     {
         int D = dense_tail < 0 ? choose_dense_tail(S) : dense_tail;
         D = std::max(0, std::min({D, n, kMaxDenseTail}));
         S.dtail = D;
         S.k0 = n - D;
+    }
+
+    // Packed strict L, update segments and their relative slots (16 bit),
+    // built through a row -> slot table of the current column.
+    S.lp.assign(n + 1, 0);
+    for (int k = 0; k < n; k++) S.lp[k + 1] = S.lp[k] + (S.cp[k + 1] - S.dg[k] - 1);
+    S.seg.clear();
+    S.seg_ptr.clear();
+    S.rel.clear();
+    S.rel_ptr.clear();
+    if (S.max_col <= 65535) {
+        // joined[j]: columns j - 1 and j belong to one supernode.
+        std::vector<char> joined(n, 0);
+        for (int j = 1; j < n; j++) {
+            const int a0 = S.dg[j - 1] + 1, la = S.cp[j] - a0, b0 = S.dg[j] + 1, lb = S.cp[j + 1] - b0;
+            joined[j] = la == lb + 1 && S.ri[a0] == j && std::equal(S.ri.begin() + b0, S.ri.begin() + b0 + lb, S.ri.begin() + a0 + 1);
+        }
+        S.seg_ptr.assign(n + 1, 0);
+        S.rel_ptr.assign(n + 1, 0);
+        std::vector<int> at(n, -1);
+        bool closed = true;
+        for (int k = 0; k < n && closed; k++) {
+            S.seg_ptr[k] = (int)(S.seg.size() / 4);
+            S.rel_ptr[k] = (long long)S.rel.size();
+            for (int p = S.cp[k]; p < S.cp[k + 1]; p++) at[S.ri[p]] = p - S.cp[k];
+            for (int p = S.cp[k]; p < S.dg[k] && S.ri[p] < S.k0;) {
+                const int j = S.ri[p];
+                int w = 1;
+                while (w < kMaxSegment && p + w < S.dg[k] && S.ri[p + w] == j + w && j + w < S.k0 && joined[j + w]) w++;
+                S.seg.push_back(j);
+                S.seg.push_back((p - S.cp[k]) | (w << 16));
+                S.seg.push_back(S.lp[j]);
+                S.seg.push_back(S.lp[j + 1] - S.lp[j]);
+                for (int t = S.dg[j] + 1; t < S.cp[j + 1]; t++) {
+                    const int s = at[S.ri[t]];
+                    if (s < 0) closed = false;   // pattern not closed under the updates
+                    S.rel.push_back((uint16_t)s);
+                }
+                p += w;
+            }
+            for (int p = S.cp[k]; p < S.cp[k + 1]; p++) at[S.ri[p]] = -1;
+        }
+        S.seg_ptr[n] = (int)(S.seg.size() / 4);
+        S.rel_ptr[n] = (long long)S.rel.size();
+        if (!closed) {
+            S.seg.clear();
+            S.seg_ptr.clear();
+            S.rel.clear();
+            S.rel_ptr.clear();
+        }
     }
 
     // Row-major copies of strict L and strict U.  Entries inside the dense
