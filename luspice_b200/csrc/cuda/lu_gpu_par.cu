@@ -6,38 +6,45 @@
 // the columns j < k that update it are discovered as a bitmap over pivot
 // positions: A(:,k) seeds the bits of its pivoted rows, and every column
 // applied sets the bits of the pivoted rows it touches (always at positions
-// above the current one).  Warp 0 finds the lowest set bit with ballots, so
-// the updates are applied in ascending pivot order, exactly the order of
-// the single-thread reference kernel (src/lu_gpu.cu:64-77); exact zeros skip
-// their column as there.  Pivot search, U and L extraction are block-wide
-// ordered compactions over the row index, giving the same entry order as the
-// single-thread kernel.  Multiply and subtract are separately rounded.
+// above the current one).  The lowest set bit is found with ballots, so the
+// updates are applied in ascending pivot order, exactly the order of the
+// single-thread reference kernel (src/lu_gpu.cu:64-77); exact zeros skip
+// their column as there.  A second bitmap holds the touched rows: pivot
+// search, U and L extraction walk it in row order (as a list, a lane per
+// row), giving the same entry order as the single-thread kernel, and never
+// look at the other rows.  Multiply and subtract are separately rounded.
+//
+// What bounds it: the serial chain of columns and of the dependencies inside
+// one, each a few dependent loads and some hundred instructions of one warp.
+// Circuit columns touch some tens of rows, so warp 0 walks them alone (no CTA
+// barrier), the next column's input and the next dependency's pointers loaded
+// ahead; the other warps join only for an update of more than kLongColumn
+// rows.  The row permutation is kept in shared memory (16 bits: n is below
+// 19,400 there).  n = 989 circuit, B200, factor and solve: 8.15 -> 5.48 ms
+// against a CTA-wide scan of all n rows per column (factor 4.92, solve 0.55
+// ms; a lane walking its word of the bitmap instead of the list: 6.85 ms).
 #include <cuda_runtime.h>
 
+#include "common.cuh"
 #include "lu_gpu_par.h"
 
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
 
-// Exclusive block scan of 0/1 flags in thread order; returns the prefix and
-// writes the total to *total (all threads).
-__device__ __forceinline__ int block_flag_scan(bool flag, int* wsum, int* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned b = __ballot_sync(0xffffffffu, flag);
-    const int before = __popc(b & ((1u << lane) - 1u));
-    __syncthreads();
-    if (lane == 0) wsum[warp] = __popc(b);
-    __syncthreads();
-    int off = 0, tot = 0;
-    for (int w = 0; w < kWarps; w++) {
-        const int c = wsum[w];
-        if (w < warp) off += c;
-        tot += c;
+// Rows of an update above which all warps share it.
+constexpr int kLongColumn = 256;
+constexpr unsigned short kNone = 0xffffu;
+
+// Inclusive prefix sum over a warp.
+__device__ __forceinline__ int warp_scan(int v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
     }
-    *total = tot;
-    return off + before;
+    return v;
 }
 
 }  // namespace
@@ -53,184 +60,319 @@ lu_factor_par_kernel(int n, const int* Ap, const int* Ai, const double* Ax, cons
         return;
     }
     extern __shared__ __align__(16) unsigned char lupar_smem[];
-    double* x = (double*)lupar_smem;                       // [n]
-    unsigned* cand = (unsigned*)(x + n);                    // [ceil(n/32)] within the 4n region
-    __shared__ int wsum[kWarps];
-    __shared__ double red_v[kWarps];
-    __shared__ int red_i[kWarps];
-    __shared__ int s_j, s_ipiv, s_status;
-    __shared__ double s_pivot;
+    __shared__ int s_beg, s_end, s_status;      // an update shared by all warps (s_beg < 0: none left)
+    __shared__ double s_xr;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nwords = (n + 31) >> 5;
+    double* x = (double*)lupar_smem;                                   // [n]
+    unsigned* cand = (unsigned*)(x + n);                               // [nwords] dependencies, by pivot position
+    unsigned* touched = cand + nwords;                                 // [nwords] rows of the column
+    unsigned short* pos = (unsigned short*)(touched + nwords);         // [n] pivot position or kNone
+    unsigned short* list = pos + n;                                    // [ncap] touched rows, ascending
+    const int ncap = (int)((LU_PAR_SHARED_BYTES(n) - (size_t)((unsigned char*)list - lupar_smem)) / 2);
     int* rowat = xi;
 
     for (int i = tid; i < n; i += kThreads) {
         x[i] = 0.0;
         pinv[i] = -1;
         rowat[i] = -1;
+        pos[i] = kNone;
     }
-    for (int w = tid; w < nwords; w += kThreads) cand[w] = 0u;
+    for (int w = tid; w < 2 * nwords; w += kThreads) cand[w] = 0u;
     if (tid == 0) s_status = -1;
     __syncthreads();
 
+    // x -= L(:,j) xr over entries [p0, p1), every stride-th from p0 + first.
+    auto update = [&](int p0, int p1, double xr, int first, int stride) {
+        for (int p = p0 + first; p < p1; p += stride) {
+            const int i = Li[p];
+            x[i] = __dsub_rn(x[i], __dmul_rn(Lx[p], xr));
+            atomicOr(touched + (i >> 5), 1u << (i & 31));
+            const int J = pos[i];
+            if (J != kNone) atomicOr(cand + (J >> 5), 1u << (J & 31));
+        }
+    };
+
     long lnz = 0, unz = 0;
-    for (int k = 0; k < n; k++) {
-        if (tid == 0) {
-            Lp[k] = (int)lnz;
-            Up[k] = (int)unz;
-        }
-        // 1. x = A(:,k) (assignment, the last duplicate wins) and seeds.
-        const int a0 = Ap[k], a1 = Ap[k + 1];
-        for (int p = a0 + tid; p < a1; p += kThreads) {
-            const int i = Ai[p];
-            bool last = true;
-            for (int p2 = p + 1; p2 < a1; p2++)
-                if (Ai[p2] == i) { last = false; break; }
-            if (last) x[i] = Ax[p];
-            const int J = pinv[i];
-            if (J >= 0) atomicOr(&cand[J >> 5], 1u << (J & 31));
-        }
-        __syncthreads();
-        // 2. Left-looking updates in ascending pivot position.
-        int cur = 0;
-        while (true) {
-            if (warp == 0) {
-                int found = -1;
-                for (int w0 = cur >> 5; w0 < nwords && found < 0; w0 += 32) {
-                    const int w = w0 + lane;
-                    unsigned bits = (w < nwords) ? cand[w] : 0u;
-                    if (w == (cur >> 5)) bits &= ~((1u << (cur & 31)) - 1u);
+    if (warp == 0) {
+        int status = -1;
+        // Column k's input: bounds, diagonal row and this lane's first entry.
+        int na0 = 0, na1 = 0, nck = 0, ni = -1;
+        double nx = 0.0;
+        int fb = 0, fe = 0, fd = 0;      // bounds and diagonal rows of 32 columns
+        auto fetch = [&](int k) {
+            if (k >= n) return;
+            if ((k & 31) == 0 && k + lane < n) {
+                fb = Ap[k + lane];
+                fe = Ap[k + lane + 1];
+                fd = diagrow[k + lane];
+            }
+            na0 = __shfl_sync(0xffffffffu, fb, k & 31);
+            na1 = __shfl_sync(0xffffffffu, fe, k & 31);
+            nck = __shfl_sync(0xffffffffu, fd, k & 31);
+            ni = na0 + lane < na1 ? Ai[na0 + lane] : -1;
+            nx = na0 + lane < na1 ? Ax[na0 + lane] : 0.0;
+        };
+        fetch(0);
+        for (int k = 0; k < n; k++) {
+            if (lane == 0) {
+                Lp[k] = (int)lnz;
+                Up[k] = (int)unz;
+            }
+            // 1. x = A(:,k) (assignment, the last duplicate wins) and seeds,
+            //    the first 32 entries loaded a column ahead.
+            const int a0 = na0, a1 = na1, ck = nck, mi = ni;
+            const double mx = nx;
+            fetch(k + 1);
+            {
+                const bool in = a0 + lane < a1;
+                const unsigned same = __match_any_sync(0xffffffffu, in ? mi : -1 - lane);
+                bool last = in && (same >> lane) == 1u;
+                for (int p = a0 + 32; p < a1 && last; p++) last = Ai[p] != mi;
+                if (last) x[mi] = mx;
+                if (in) {
+                    atomicOr(touched + (mi >> 5), 1u << (mi & 31));
+                    const int J = pos[mi];
+                    if (J != kNone) atomicOr(cand + (J >> 5), 1u << (J & 31));
+                }
+            }
+            for (int p = a0 + 32 + lane; p < a1; p += 32) {
+                const int i = Ai[p];
+                bool last = true;
+                for (int p2 = p + 1; p2 < a1; p2++)
+                    if (Ai[p2] == i) { last = false; break; }
+                if (last) x[i] = Ax[p];
+                atomicOr(touched + (i >> 5), 1u << (i & 31));
+                const int J = pos[i];
+                if (J != kNone) atomicOr(cand + (J >> 5), 1u << (J & 31));
+            }
+            __syncwarp();
+            // 2. Left-looking updates in ascending pivot position; the
+            //    pointers of the next dependency known so far are loaded
+            //    beside the current update.
+            int pj = -1, pp0 = 0, pp1 = 0, prow = 0;
+            for (int w0 = 0; w0 < nwords; w0 += 32) {
+                const int w = w0 + lane;
+                while (true) {
+                    const unsigned bits = w < nwords ? cand[w] : 0u;
                     const unsigned any = __ballot_sync(0xffffffffu, bits != 0u);
-                    if (any) {
-                        const int src = __ffs(any) - 1;
-                        const unsigned wb = __shfl_sync(0xffffffffu, bits, src);
-                        found = ((w0 + src) << 5) + (__ffs(wb) - 1);
+                    if (!any) break;
+                    const int src = __ffs(any) - 1;
+                    const unsigned wb = __shfl_sync(0xffffffffu, bits, src);
+                    const int j = ((w0 + src) << 5) + (__ffs(wb) - 1);
+                    if (j != pj) {
+                        pp0 = Lp[j] + 1;
+                        pp1 = Lp[j + 1];
+                        prow = rowat[j];
                     }
-                }
-                if (lane == 0) {
-                    s_j = found;
-                    if (found >= 0) cand[found >> 5] &= ~(1u << (found & 31));
-                }
-            }
-            __syncthreads();
-            const int j = s_j;
-            if (j < 0) break;
-            const double xr = x[rowat[j]];
-            if (xr != 0.0) {
-                for (int p = Lp[j] + 1 + tid; p < Lp[j + 1]; p += kThreads) {
-                    const int i = Li[p];
-                    x[i] = __dsub_rn(x[i], __dmul_rn(Lx[p], xr));
-                    const int J = pinv[i];
-                    if (J >= 0) atomicOr(&cand[J >> 5], 1u << (J & 31));
-                }
-            }
-            cur = j + 1;
-            __syncthreads();
-        }
-        // 3. Pivot search (largest |x|, smallest row on ties) and U(:,k).
-        double bv = -1.0;
-        int bi = -1;
-        for (int base = 0; base < n; base += kThreads) {
-            const int i = base + tid;
-            bool isU = false;
-            double xi_v = 0.0;
-            int pi = -1;
-            if (i < n) {
-                pi = pinv[i];
-                xi_v = x[i];
-                if (pi < 0) {
-                    const double t = fabs(xi_v);
-                    if (t > bv) { bv = t; bi = i; }
-                } else {
-                    isU = xi_v != 0.0;
+                    const int p0 = pp0, p1 = pp1;
+                    const double xr = x[prow];
+                    // The next set bit: in this word or the next non-empty one.
+                    const unsigned rest = wb & (wb - 1u), more = any & (any - 1u);
+                    const int nsrc = rest ? src : __ffs(more) - 1;
+                    const unsigned nb = __shfl_sync(0xffffffffu, bits, nsrc < 0 ? 0 : nsrc);
+                    pj = rest ? ((w0 + src) << 5) + (__ffs(rest) - 1)
+                              : nsrc >= 0 ? ((w0 + nsrc) << 5) + (__ffs(nb) - 1) : -1;
+                    if (pj >= 0) {
+                        pp0 = Lp[pj] + 1;
+                        pp1 = Lp[pj + 1];
+                        prow = rowat[pj];
+                    }
+                    __syncwarp();
+                    if (lane == src) cand[w] = rest;
+                    __syncwarp();
+                    if (xr != 0.0) {
+                        if (p1 - p0 <= kLongColumn) {
+                            update(p0, p1, xr, lane, 32);
+                        } else {
+                            if (lane == 0) {
+                                s_beg = p0;
+                                s_end = p1;
+                                s_xr = xr;
+                            }
+                            __syncthreads();
+                            update(p0, p1, xr, tid, kThreads);
+                            __syncthreads();
+                        }
+                    }
+                    __syncwarp();
                 }
             }
-            int tot;
-            const int off = block_flag_scan(isU, wsum, &tot);
-            if (unz + tot > Ucap) {
-                if (tid == 0) s_status = -2;
-            } else if (isU) {
-                Ui[unz + off] = pi;
-                Ux[unz + off] = xi_v;
+            // 3. The touched rows as an ascending list, a lane per row from
+            //    here on (columns that touch more rows than the list holds
+            //    walk the bitmap, a lane per word).
+            int rows = 0;
+            for (int w0 = 0; w0 < nwords; w0 += 32) {
+                const int w = w0 + lane;
+                const unsigned bits = w < nwords ? touched[w] : 0u;
+                const int inc = warp_scan(__popc(bits));
+                int o = rows + inc - __popc(bits);
+                rows += __shfl_sync(0xffffffffu, inc, 31);
+                if (rows <= ncap)
+                    for (unsigned b = bits; b; b &= b - 1u) list[o++] = (unsigned short)((w << 5) + __ffs(b) - 1);
             }
-            unz += tot;
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            const double v2 = __shfl_down_sync(0xffffffffu, bv, o);
-            const int i2 = __shfl_down_sync(0xffffffffu, bi, o);
-            if (v2 > bv || (v2 == bv && i2 >= 0 && (bi < 0 || i2 < bi))) { bv = v2; bi = i2; }
-        }
-        if (lane == 0) { red_v[warp] = bv; red_i[warp] = bi; }
-        __syncthreads();
-        if (tid == 0) {
-            double a = -1.0;
-            int ip = -1;
-            for (int w = 0; w < kWarps; w++) {
-                const double v2 = red_v[w];
-                const int i2 = red_i[w];
-                if (v2 > a || (v2 == a && i2 >= 0 && (ip < 0 || i2 < ip))) { a = v2; ip = i2; }
-            }
-            if (s_status == -1) {
-                if (ip == -1 || a <= 0.0) {
-                    s_status = k;
-                } else {
-                    const int ck = diagrow[k];
-                    if (pinv[ck] < 0 && fabs(x[ck]) >= a) ip = ck;
-                    s_ipiv = ip;
-                    s_pivot = x[ip];
-                    if (unz + 1 > Ucap || lnz + 1 > Lcap) {
-                        s_status = -2;
+            __syncwarp();
+            const bool listed = rows <= ncap;
+            const unsigned below = (1u << lane) - 1u;
+            // 4. Pivot search (largest |x|, smallest row on ties) and U(:,k),
+            //    rows in ascending order.
+            double bv = -1.0;
+            int bi = -1;
+            if (listed) {
+                for (int t = 0; t < rows; t += 32) {
+                    const int i = t + lane < rows ? list[t + lane] : -1;
+                    const double v = i >= 0 ? x[i] : 0.0;
+                    const int J = i >= 0 ? pos[i] : kNone;
+                    const bool isU = J != kNone && v != 0.0;
+                    if (i >= 0 && J == kNone && fabs(v) > bv) { bv = fabs(v); bi = i; }
+                    const unsigned m = __ballot_sync(0xffffffffu, isU);
+                    const int tot = __popc(m);
+                    if (unz + tot > Ucap) {
+                        status = -2;
+                    } else if (isU) {
+                        const long o = unz + __popc(m & below);
+                        Ui[o] = J;
+                        Ux[o] = v;
+                    }
+                    unz += tot;
+                }
+            } else {
+                for (int w0 = 0; w0 < nwords; w0 += 32) {
+                    const int w = w0 + lane;
+                    const unsigned bits = w < nwords ? touched[w] : 0u;
+                    int cnt = 0;
+                    for (unsigned b = bits; b; b &= b - 1u) {
+                        const int i = (w << 5) + __ffs(b) - 1;
+                        const double v = x[i];
+                        if (pos[i] == kNone) {
+                            const double t = fabs(v);
+                            if (t > bv) { bv = t; bi = i; }
+                        } else if (v != 0.0) {
+                            cnt++;
+                        }
+                    }
+                    const int inc = warp_scan(cnt);
+                    const int tot = __shfl_sync(0xffffffffu, inc, 31);
+                    if (unz + tot > Ucap) {
+                        status = -2;
                     } else {
-                        Ui[unz] = k;
-                        Ux[unz] = s_pivot;
-                        pinv[ip] = k;
-                        rowat[k] = ip;
-                        Li[lnz] = ip;
-                        Lx[lnz] = 1.0;
+                        long o = unz + inc - cnt;
+                        for (unsigned b = bits; b && cnt > 0; b &= b - 1u) {
+                            const int i = (w << 5) + __ffs(b) - 1;
+                            const double v = x[i];
+                            const int J = pos[i];
+                            if (J != kNone && v != 0.0) {
+                                Ui[o] = J;
+                                Ux[o] = v;
+                                o++;
+                            }
+                        }
                     }
+                    unz += tot;
                 }
             }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double v2 = __shfl_xor_sync(0xffffffffu, bv, o);
+                const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (v2 > bv || (v2 == bv && i2 >= 0 && (bi < 0 || i2 < bi))) { bv = v2; bi = i2; }
+            }
+            if (status != -1) break;
+            if (bi == -1 || bv <= 0.0) { status = k; break; }
+            if (pos[ck] == kNone && fabs(x[ck]) >= bv) bi = ck;
+            if (unz + 1 > Ucap || lnz + 1 > Lcap) { status = -2; break; }
+            const double pivot = x[bi], rpivot = __drcp_rn(pivot);
+            __syncwarp();
+            if (lane == 0) {
+                Ui[unz] = k;
+                Ux[unz] = pivot;
+                pinv[bi] = k;
+                pos[bi] = (unsigned short)k;
+                rowat[k] = bi;
+                Li[lnz] = bi;
+                Lx[lnz] = 1.0;
+            }
+            __syncwarp();
+            unz += 1;
+            lnz += 1;
+            // 5. L(:,k): unpivoted nonzero rows ascending, scaled by the
+            //    pivot; the work vector and the bitmap are cleared on the way.
+            if (listed) {
+                for (int t = 0; t < rows; t += 32) {
+                    const int i = t + lane < rows ? list[t + lane] : -1;
+                    const double v = i >= 0 ? x[i] : 0.0;
+                    const bool isL = i >= 0 && pos[i] == kNone && v != 0.0;
+                    const unsigned m = __ballot_sync(0xffffffffu, isL);
+                    const int tot = __popc(m);
+                    if (lnz + tot > Lcap) {
+                        status = -2;
+                    } else if (isL) {
+                        const long o = lnz + __popc(m & below);
+                        Li[o] = i;
+                        Lx[o] = lusp::div_by<false>(v, pivot, rpivot);
+                    }
+                    if (i >= 0) {
+                        x[i] = 0.0;
+                        touched[i >> 5] = 0u;
+                    }
+                    lnz += tot;
+                }
+            } else {
+                for (int w0 = 0; w0 < nwords; w0 += 32) {
+                    const int w = w0 + lane;
+                    const unsigned bits = w < nwords ? touched[w] : 0u;
+                    int cnt = 0;
+                    for (unsigned b = bits; b; b &= b - 1u) {
+                        const int i = (w << 5) + __ffs(b) - 1;
+                        cnt += pos[i] == kNone && x[i] != 0.0;
+                    }
+                    const int inc = warp_scan(cnt);
+                    const int tot = __shfl_sync(0xffffffffu, inc, 31);
+                    const bool fits = lnz + tot <= Lcap;
+                    if (!fits) status = -2;
+                    long o = lnz + inc - cnt;
+                    for (unsigned b = bits; b; b &= b - 1u) {
+                        const int i = (w << 5) + __ffs(b) - 1;
+                        const double v = x[i];
+                        x[i] = 0.0;
+                        if (fits && pos[i] == kNone && v != 0.0) {
+                            Li[o] = i;
+                            Lx[o] = lusp::div_by<false>(v, pivot, rpivot);
+                            o++;
+                        }
+                    }
+                    if (w < nwords) touched[w] = 0u;
+                    lnz += tot;
+                }
+            }
+            __syncwarp();
+            if (status != -1) break;
+            // The next column's reads see this one's entries and pointers.
+            if (lane == 0) Lp[k + 1] = (int)lnz;
+            __syncwarp();
+        }
+        if (lane == 0) {
+            s_beg = -1;
+            s_status = status;
+            if (status == -1) Up[n] = (int)unz;
         }
         __syncthreads();
-        if (s_status != -1) {
-            if (tid == 0) *singular_out = s_status;
-            return;
-        }
-        unz += 1;
-        lnz += 1;
-        // 4. L(:,k): unpivoted nonzero rows ascending, scaled by the pivot;
-        //    the work vector is cleared on the way.
-        const double pivot = s_pivot;
-        for (int base = 0; base < n; base += kThreads) {
-            const int i = base + tid;
-            bool isL = false;
-            double v = 0.0;
-            if (i < n) {
-                v = x[i];
-                isL = pinv[i] < 0 && v != 0.0;
-                x[i] = 0.0;
-            }
-            int tot;
-            const int off = block_flag_scan(isL, wsum, &tot);
-            if (lnz + tot > Lcap) {
-                if (tid == 0) s_status = -2;
-            } else if (isL) {
-                Li[lnz + off] = i;
-                Lx[lnz + off] = __ddiv_rn(v, pivot);
-            }
-            lnz += tot;
-        }
-        __syncthreads();
-        if (s_status != -1) {
-            if (tid == 0) *singular_out = s_status;
-            return;
+        unz = __shfl_sync(0xffffffffu, unz, 0);
+    } else {
+        while (true) {
+            __syncthreads();
+            const int beg = s_beg;
+            if (beg < 0) break;
+            update(beg, s_end, s_xr, tid, kThreads);
+            __syncthreads();
         }
     }
-    if (tid == 0) {
-        Lp[n] = (int)lnz;
-        Up[n] = (int)unz;
+    if (s_status != -1) {
+        if (tid == 0) *singular_out = s_status;
+        return;
     }
-    for (long p = tid; p < lnz; p += kThreads) Li[p] = pinv[Li[p]];
+    const int total = Lp[n];
+    for (int p = tid; p < total; p += kThreads) Li[p] = pinv[Li[p]];
     __syncthreads();
     if (tid == 0) {
         *lnnz = (int)lnz;
@@ -239,16 +381,85 @@ lu_factor_par_kernel(int n, const int* Ap, const int* Ai, const double* Ax, cons
     }
 }
 
+// One column sweep of trisolve over v (shared memory) by one warp.  UPPER:
+// columns from the last down, v[k] = v[k] / diagonal (the column's last entry);
+// else from the first up (the first entry), in both v[i] -= entry * v[k] for
+// the column's other entries, separately rounded.  The pointers of 32 columns
+// are loaded together, a column's first 32 entries and its diagonal four
+// columns ahead, so the chain of a column is the shared-memory round trip of v
+// and the update.
+template <bool UPPER>
+__device__ void trisolve_sweep(int n, const int* cp, const int* ci, const double* cx, double* v) {
+    const int lane = threadIdx.x & 31;
+    int pb = 0, pe = 0;                     // pointers of column (32 block + lane) in sweep order
+    auto bounds = [&](int t, int& p0, int& p1) {   // t-th column of the sweep (t < n)
+        if ((t & 31) == 0) {
+            const int k = UPPER ? n - 1 - t - lane : t + lane;
+            if (k >= 0 && k < n) {
+                pb = cp[k];
+                pe = cp[k + 1];
+            }
+        }
+        p0 = __shfl_sync(0xffffffffu, pb, t & 31);
+        p1 = __shfl_sync(0xffffffffu, pe, t & 31);
+    };
+    // Entries beside the diagonal: [p0 + 1, p1) of L, [p0, p1 - 1) of U, of
+    // the next kAhead columns.
+    constexpr int kAhead = 4;
+    int p0[kAhead], p1[kAhead], i[kAhead];
+    double e[kAhead], dg[kAhead];
+    auto fetch = [&](int t, int u) {
+        bounds(t, p0[u], p1[u]);
+        const int q = UPPER ? p0[u] + lane : p0[u] + 1 + lane, end = UPPER ? p1[u] - 1 : p1[u];
+        i[u] = q < end ? ci[q] : -1;
+        e[u] = q < end ? cx[q] : 0.0;
+        dg[u] = cx[UPPER ? p1[u] - 1 : p0[u]];
+    };
+#pragma unroll
+    for (int u = 0; u < kAhead; u++)
+        if (u < n) fetch(u, u);
+    double rd = n > 0 ? __drcp_rn(dg[0]) : 1.0;
+    for (int t0 = 0; t0 < n; t0 += kAhead) {
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) {
+            const int t = t0 + u;
+            if (t >= n) break;
+            const int k = UPPER ? n - 1 - t : t;
+            const double d = dg[u], r = rd;
+            const double vk = d == 1.0 ? v[k] : lusp::div_by<false>(v[k], d, r);
+            __syncwarp();
+            if (lane == 0) v[k] = vk;
+            if (i[u] >= 0) v[i[u]] = __dsub_rn(v[i[u]], __dmul_rn(e[u], vk));
+            const int end = UPPER ? p1[u] - 1 : p1[u];
+            for (int q = (UPPER ? p0[u] : p0[u] + 1) + 32 + lane; q < end; q += 32) {
+                const int i2 = ci[q];
+                v[i2] = __dsub_rn(v[i2], __dmul_rn(cx[q], vk));
+            }
+            if (t + kAhead < n) fetch(t + kAhead, u);
+            if (t + 1 < n && dg[(u + 1) % kAhead] != 1.0) rd = __drcp_rn(dg[(u + 1) % kAhead]);
+            __syncwarp();
+        }
+    }
+}
+
+// Systems whose solve vector fits the kernel's static shared memory.
+constexpr int kTriShared = 6000;
+
 // pb = P b; L y = pb by columns (unit diagonal first); U z = y by columns
 // (diagonal last); x = Q z.  Same operation sequence as splu.h:210-239, so
-// the result is bitwise that of the host solve on the same factors.
+// the result is bitwise that of the host solve on the same factors.  Serial
+// over columns; up to kTriShared unknowns one warp walks them on a vector in
+// shared memory (a column costs its few dependent shared-memory accesses, no
+// CTA barrier and no global round trip), larger systems with the whole CTA on
+// the caller's work arrays.
 __global__ void __launch_bounds__(256)
 trisolve_par_kernel(int n, const int* Lp, const int* Li, const double* Lx, const int* Up,
                     const int* Ui, const double* Ux, const int* pinv, const int* q,
                     const double* b, double* x, int* work_i, double* work_d) {
+    __shared__ double sv[kTriShared];
     const int tid = threadIdx.x, nt = blockDim.x;
     int* rowat = work_i;
-    double* pb = work_d;
+    double* pb = n <= kTriShared ? sv : work_d;
     double* y = work_d + n;
     for (int i = tid; i < n; i += nt) rowat[i] = -1;
     __syncthreads();
@@ -257,6 +468,15 @@ trisolve_par_kernel(int n, const int* Lp, const int* Li, const double* Lx, const
     __syncthreads();
     for (int k = tid; k < n; k += nt) pb[k] = rowat[k] >= 0 ? b[rowat[k]] : 0.0;
     __syncthreads();
+    if (n <= kTriShared) {
+        if (tid < 32) {
+            trisolve_sweep<false>(n, Lp, Li, Lx, sv);
+            trisolve_sweep<true>(n, Up, Ui, Ux, sv);
+        }
+        __syncthreads();
+        for (int k = tid; k < n; k += nt) x[q ? q[k] : k] = sv[k];
+        return;
+    }
     for (int k = 0; k < n; k++) {
         const double yk = __ddiv_rn(pb[k], Lx[Lp[k]]);
         if (tid == 0) y[k] = yk;
