@@ -64,36 +64,49 @@ template <> __device__ __forceinline__ double ldv<__half>(const __half* p) {
     return (double)__half2float(__ldg(p));
 }
 
-// Blocks [0, sell_blocks) take the slices; the blocks after them take the
-// long rows, a warp per row (lanes over its entries, four partial sums per
-// lane, a fixed-order warp reduction).
-template <int C, typename VT>
+// Blocks [0, sell_blocks) take the slices, a warp each; the blocks after them
+// take the long rows, a block per row (fixed-order reduction): a supply net's
+// row of 800 entries is then one round of loads, where a warp walking it
+// (seven rounds of four loads a lane) was the whole launch.  n = 40,000 circuit
+// with four such rows, fp32, B200: 8.2 -> 6.1 us a product.
+// WIDE (all warps resident at once, so a warp's latency is the launch's): row
+// numbers and up to eight entries per lane requested before the first is
+// used: 6.1 -> 4.1 us there.  Larger matrices stream (a mesh of 2 M nodes, fp64,
+// at 4.1 TB/s) and are 0.8 % slower that way (two or four slices per warp: 11 %).
+template <int C, bool WIDE, typename VT>
 __global__ void __launch_bounds__(256)
 sell_kernel(int nslices, const int* __restrict__ ptr, const int* __restrict__ col,
             const VT* __restrict__ val, const int* __restrict__ perm,
             const double* __restrict__ x, double* __restrict__ y,
-            const double* __restrict__ row_div, int sell_blocks, int nlong,
+            const double* __restrict__ row_div, int sell_blocks,
             const int* __restrict__ lrow, const int* __restrict__ lptr, const int* __restrict__ lcol,
             const VT* __restrict__ lval) {
     if ((int)blockIdx.x >= sell_blocks) {
-        const int lane = threadIdx.x & 31;
-        const int w = ((blockIdx.x - sell_blocks) * blockDim.x + threadIdx.x) >> 5;
-        if (w >= nlong) return;
+        __shared__ double part[8];
+        const int w = (int)blockIdx.x - sell_blocks;
         const int p1 = lptr[w + 1];
         double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-        int p = lptr[w] + lane;
-        for (; p + 96 < p1; p += 128) {
-            const int c0 = lcol[p], c1 = lcol[p + 32], c2 = lcol[p + 64], c3 = lcol[p + 96];
+        int p = lptr[w] + (int)threadIdx.x;
+        for (; p + 768 < p1; p += 1024) {
+            const int c0 = lcol[p], c1 = lcol[p + 256], c2 = lcol[p + 512], c3 = lcol[p + 768];
             a0 = fma(ldv<VT>(lval + p), __ldg(x + c0), a0);
-            a1 = fma(ldv<VT>(lval + p + 32), __ldg(x + c1), a1);
-            a2 = fma(ldv<VT>(lval + p + 64), __ldg(x + c2), a2);
-            a3 = fma(ldv<VT>(lval + p + 96), __ldg(x + c3), a3);
+            a1 = fma(ldv<VT>(lval + p + 256), __ldg(x + c1), a1);
+            a2 = fma(ldv<VT>(lval + p + 512), __ldg(x + c2), a2);
+            a3 = fma(ldv<VT>(lval + p + 768), __ldg(x + c3), a3);
         }
-        for (; p < p1; p += 32) a0 = fma(ldv<VT>(lval + p), __ldg(x + lcol[p]), a0);
+        // At most three entries per thread are left.
+        const bool b0 = p < p1, b1 = p + 256 < p1, b2 = p + 512 < p1;
+        const int c0 = b0 ? lcol[p] : 0, c1 = b1 ? lcol[p + 256] : 0, c2 = b2 ? lcol[p + 512] : 0;
+        if (b0) a0 = fma(ldv<VT>(lval + p), __ldg(x + c0), a0);
+        if (b1) a1 = fma(ldv<VT>(lval + p + 256), __ldg(x + c1), a1);
+        if (b2) a2 = fma(ldv<VT>(lval + p + 512), __ldg(x + c2), a2);
         double acc = (a0 + a1) + (a2 + a3);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) {
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            acc = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
             const int row = lrow[w];
             y[row] = row_div ? acc / row_div[row] : acc;
         }
@@ -106,25 +119,58 @@ sell_kernel(int nslices, const int* __restrict__ ptr, const int* __restrict__ co
     const int r = lane % C, sub = lane / C;
     const int base = ptr[s];
     const int L = (ptr[s + 1] - base) / C;
+    int row = -1;
+    if (WIDE && sub == 0) row = perm[s * C + r];
     double acc = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    int t = sub;
-    for (; t + 3 * G < L; t += 4 * G) {
-        const int e = base + t * C + r, d = G * C;
-        const int c0 = col[e], c1 = col[e + d], c2 = col[e + 2 * d], c3 = col[e + 3 * d];
-        acc = fma(ldv<VT>(val + e), __ldg(x + c0), acc);
-        a1 = fma(ldv<VT>(val + e + d), __ldg(x + c1), a1);
-        a2 = fma(ldv<VT>(val + e + 2 * d), __ldg(x + c2), a2);
-        a3 = fma(ldv<VT>(val + e + 3 * d), __ldg(x + c3), a3);
-    }
-    for (; t < L; t += G) {
-        const int e = base + t * C + r;
-        acc = fma(ldv<VT>(val + e), __ldg(x + col[e]), acc);
+    if (WIDE) {
+        // The same sums as below: four interleaved partial sums over groups
+        // of four, the rest into the first.
+        for (int t = sub; t < L; t += 8 * G) {
+            int c[8];
+            double v[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const bool in = t + q * G < L;
+                const int e = base + (t + q * G) * C + r;
+                c[q] = in ? col[e] : 0;
+                v[q] = in ? ldv<VT>(val + e) : 0.0;
+            }
+#pragma unroll
+            for (int h = 0; h < 8; h += 4) {
+                if (t + (h + 3) * G < L) {
+                    const double x0 = __ldg(x + c[h]), x1 = __ldg(x + c[h + 1]);
+                    const double x2 = __ldg(x + c[h + 2]), x3 = __ldg(x + c[h + 3]);
+                    acc = fma(v[h], x0, acc);
+                    a1 = fma(v[h + 1], x1, a1);
+                    a2 = fma(v[h + 2], x2, a2);
+                    a3 = fma(v[h + 3], x3, a3);
+                } else {
+#pragma unroll
+                    for (int q = h; q < h + 3; q++)
+                        if (t + q * G < L) acc = fma(v[q], __ldg(x + c[q]), acc);
+                }
+            }
+        }
+    } else {
+        int t = sub;
+        for (; t + 3 * G < L; t += 4 * G) {
+            const int e = base + t * C + r, d = G * C;
+            const int c0 = col[e], c1 = col[e + d], c2 = col[e + 2 * d], c3 = col[e + 3 * d];
+            acc = fma(ldv<VT>(val + e), __ldg(x + c0), acc);
+            a1 = fma(ldv<VT>(val + e + d), __ldg(x + c1), a1);
+            a2 = fma(ldv<VT>(val + e + 2 * d), __ldg(x + c2), a2);
+            a3 = fma(ldv<VT>(val + e + 3 * d), __ldg(x + c3), a3);
+        }
+        for (; t < L; t += G) {
+            const int e = base + t * C + r;
+            acc = fma(ldv<VT>(val + e), __ldg(x + col[e]), acc);
+        }
     }
     acc = (acc + a1) + (a2 + a3);
 #pragma unroll
     for (int o = 16; o >= C; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (sub == 0) {
-        const int row = perm[s * C + r];
+        if (!WIDE) row = perm[s * C + r];
         if (row >= 0) y[row] = row_div ? acc / row_div[row] : acc;
     }
 }
@@ -150,13 +196,34 @@ struct SellObj {
     double* d_xs = nullptr;     // fp16: scaled x
     double smin = 0, smax = 0;
     // Rows much longer than the rest (supply nets) stay out of the slices
-    // (one of them would set a whole slice's width): CSR, a warp per row.
+    // (one of them would set a whole slice's width): CSR, a block per row.
     int nlong = 0;
     int* d_lrow = nullptr;      // [nlong] row
     int* d_lptr = nullptr;      // [nlong+1]
     int* d_lcol = nullptr;
     void* d_lval = nullptr;
 };
+
+template <int C, typename VT>
+static void sell_value(const SellObj* S, int grid, int sell_blocks, bool wide, const double* x, double* y,
+                       const double* rsc, cudaStream_t st) {
+    if (wide)
+        sell_kernel<C, true, VT><<<grid, 256, 0, st>>>(S->nslices, S->d_ptr, S->d_col, (const VT*)S->d_val, S->d_perm, x, y,
+                                                      rsc, sell_blocks, S->d_lrow, S->d_lptr, S->d_lcol,
+                                                      (const VT*)S->d_lval);
+    else
+        sell_kernel<C, false, VT><<<grid, 256, 0, st>>>(S->nslices, S->d_ptr, S->d_col, (const VT*)S->d_val, S->d_perm, x, y,
+                                                       rsc, sell_blocks, S->d_lrow, S->d_lptr, S->d_lcol,
+                                                       (const VT*)S->d_lval);
+}
+
+template <int C>
+static void sell_kind(const SellObj* S, int grid, int sell_blocks, bool wide, const double* x, double* y,
+                      const double* rsc, cudaStream_t st) {
+    if (S->kind == 0) sell_value<C, double>(S, grid, sell_blocks, wide, x, y, rsc, st);
+    else if (S->kind == 1) sell_value<C, float>(S, grid, sell_blocks, wide, x, y, rsc, st);
+    else sell_value<C, __half>(S, grid, sell_blocks, wide, x, y, rsc, st);
+}
 
 // Ruiz equilibration (max norm): alternately scale rows and columns by
 // 1/sqrt(max |a|) until every row and column maximum is within tol of 1.
@@ -445,28 +512,15 @@ int lusp_sell_spmv(const lusp_sell* hs, const double* d_x, double* d_y, void* st
         xin = S->d_xs;
     }
     const int sell_blocks = (int)(((long)S->nslices * 32 + 255) / 256);
-    const int long_blocks = (int)(((long)S->nlong * 32 + 255) / 256);
-    const int grid = sell_blocks + long_blocks;
+    const int grid = sell_blocks + S->nlong;   // a block per long row
     const double* rsc = S->kind == 2 ? S->d_rs : nullptr;
-#define LUSP_SELL_CASE(CC)                                                                        \
-    if (S->C == CC) {                                                                             \
-        if (S->kind == 0)                                                                         \
-            sell_kernel<CC, double><<<grid, 256, 0, st>>>(S->nslices, S->d_ptr, S->d_col,         \
-                (const double*)S->d_val, S->d_perm, xin, d_y, rsc, sell_blocks, S->nlong,         \
-                S->d_lrow, S->d_lptr, S->d_lcol, (const double*)S->d_lval);                       \
-        else if (S->kind == 1)                                                                    \
-            sell_kernel<CC, float><<<grid, 256, 0, st>>>(S->nslices, S->d_ptr, S->d_col,          \
-                (const float*)S->d_val, S->d_perm, xin, d_y, rsc, sell_blocks, S->nlong,          \
-                S->d_lrow, S->d_lptr, S->d_lcol, (const float*)S->d_lval);                        \
-        else                                                                                      \
-            sell_kernel<CC, __half><<<grid, 256, 0, st>>>(S->nslices, S->d_ptr, S->d_col,         \
-                (const __half*)S->d_val, S->d_perm, xin, d_y, rsc, sell_blocks, S->nlong,         \
-                S->d_lrow, S->d_lptr, S->d_lcol, (const __half*)S->d_lval);                       \
+    // Wide slices while every warp is resident at once (40 per SM).
+    const bool wide = S->nslices <= 40 * lusp::sm_count();
+    if (grid > 0) {
+        if (S->C == 8) sell_kind<8>(S, grid, sell_blocks, wide, xin, d_y, rsc, st);
+        else if (S->C == 16) sell_kind<16>(S, grid, sell_blocks, wide, xin, d_y, rsc, st);
+        else sell_kind<32>(S, grid, sell_blocks, wide, xin, d_y, rsc, st);
     }
-    LUSP_SELL_CASE(8)
-    LUSP_SELL_CASE(16)
-    LUSP_SELL_CASE(32)
-#undef LUSP_SELL_CASE
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? LUSP_OK : lusp::cuda_fail(e, "sell spmv launch");
 }
