@@ -160,12 +160,11 @@ __device__ void cta_store_pivot_stats(SysStats* st, Smem& sm, double minpiv, dou
 // column engine.
 //
 // What bounds it: the chain panel -> update of the next block column ->
-// next panel.  A panel column costs one division, one barrier and the
-// pivot row's broadcast because a thread keeps its row of the panel in
-// registers (measured below); the updates run at the fp64 pipe's rate
-// because a lane keeps its column of the panel's U block in registers and
-// the multipliers are broadcast from shared memory (one 16-byte load per two
-// multiply-subtract pairs of a warp).  Warps other than the last stream
+// next panel.  A thread keeps its row of the panel in registers, so a panel
+// column reads only the pivot row from shared memory.  In the updates a lane
+// keeps its column of the panel's U block in registers and the multipliers
+// are broadcast from shared memory (one 16-byte load per two multiply-subtract
+// pairs of a warp), which takes the load pipe about twice the fp64 pipe's time.  Warps other than the last stream
 // their own rows of the panel (four rows of 256 bytes per copy group) with
 // no CTA barrier; the last warp solves the next panel's 32 x 32 unit-lower
 // block for U meanwhile.  CL: the two CTAs of a cluster take the block
@@ -356,17 +355,16 @@ __device__ __noinline__ void dense_update_rows(double* xs, const double* xk, con
 // per column instead of one).
 // ud: the pivot rows, entry (r, 4 (r / 4) + q) at ud + 34 r + q, the pivot's
 // reciprocal at ud + 34 r + 32.  vmax[c]: bits of the largest entry of column
-// c below the pivot before scaling, over the entries whose multiplier is at
-// least 1 in magnitude (the others are below the pivot, so they do not count
-// for its ratio).  Ends with a CTA barrier.
+// c below the pivot before scaling, over the entries above the pivot in
+// magnitude (the others do not count for its ratio).  Ends with a CTA barrier.
 template <typename VT>
 __device__ __noinline__ void dense_panel(double* xj, double* ud, unsigned long long* vmax, int R, int w) {
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int pw = (min(R, nt) + 31) >> 5;
     auto scale = [](double v, double p, double rp) { return (double)ValTraits<VT>::to(div_by(v, p, rp)); };
     auto sub = [](double a, double l, double u) { return __dsub_rn(a, __dmul_rn(l, u)); };
-    auto note = [&](int c, double v, double l) {
-        if (fabs(l) >= 1.0) atomicMax(vmax + c, (unsigned long long)__double_as_longlong(fabs(v)));
+    auto note = [&](int c, double v, double p) {
+        if (fabs(v) > fabs(p)) atomicMax(vmax + c, (unsigned long long)__double_as_longlong(fabs(v)));
     };
     if (tid < 32) vmax[tid] = 0ull;
     __syncthreads();
@@ -389,7 +387,7 @@ __device__ __noinline__ void dense_panel(double* xj, double* ud, unsigned long l
                 __syncwarp();
                 if (lane > c) {
                     const double l = scale(x[c], p, rp);
-                    note(c, x[c], l);
+                    note(c, x[c], p);
                     x[c] = l;
                     if (!(c & 1)) x[c + 1] = sub(x[c + 1], l, uc[c + 1]);
 #pragma unroll
@@ -448,9 +446,9 @@ __device__ __noinline__ void dense_panel(double* xj, double* ud, unsigned long l
 #pragma unroll
                 for (int k = 0; k < 4; k++) row[c + k] = l[k];
             }
-            if (r < R && fmax(fmax(fabs(l[0]), fabs(l[1])), fmax(fabs(l[2]), fabs(l[3]))) >= 1.0) {
+            if (r < R) {
 #pragma unroll
-                for (int k = 0; k < 4; k++) note(c + k, v[k], l[k]);
+                for (int k = 0; k < 4; k++) note(c + k, v[k], uc[k * 34 + k]);
             }
         }
     }
@@ -817,11 +815,12 @@ __device__ void spread_finish(const SysDev& S, unsigned* sync, int group, Smem& 
     }
 }
 
-// Cycle split of the refactor (waits for dependency columns, gathers of
-// their L parts, updates) into SysStats::cyc_wait / cyc_gather / cyc_update.
+// Cycle split of the refactor (waits for dependency columns, updates) into
+// SysStats::cyc_wait / cyc_update; cyc_gather is 0, since the L parts are read
+// by the updates themselves.
 // Reading the SM clock three times per dependency round costs ~3 % of the
 // grid refactor, so the split is a build option (-DLUSP_REFACTOR_PHASE_CYCLES=1);
-// without it the three fields stay 0 (cyc_refactor is always written).
+// without it both fields stay 0 (cyc_refactor is always written).
 #ifndef LUSP_REFACTOR_PHASE_CYCLES
 #define LUSP_REFACTOR_PHASE_CYCLES 0
 #endif
@@ -1095,9 +1094,9 @@ __device__ void refactor_phase(const RefactorCtx& cx, const SmemPlan& plan, char
         }
         const double piv = x[d], rpiv = __drcp_rn(piv);
         // The multipliers, published before anything else of the column.
-        // amax: the largest |x| below the pivot whose multiplier is at least
-        // 1 in magnitude (the others are below the pivot, so they do not
-        // count for its ratio).
+        // amax: the largest |x| below the pivot that exceeds it (the others do
+        // not count for its ratio).
+        const double ap = fabs(piv);
         double amax = 0.0;
         VT* lk = (VT*)S.lcol + rec[14] - d - 1;
 #pragma unroll 4
@@ -1106,14 +1105,13 @@ __device__ void refactor_phase(const RefactorCtx& cx, const SmemPlan& plan, char
             const VT l = ValTraits<VT>::to(div_by<false>(v, piv, rpiv));
             lk[t] = l;
             x[t] = (double)l;
-            if (fabs((double)l) >= 1.0) amax = fmax(amax, fabs(v));
+            if (fabs(v) > ap) amax = fmax(amax, fabs(v));
         }
         // Release: the column's values before its ready bit.
         share_release_t<SPREAD>(csize);
         __syncwarp();
         if (lane == 0) set_ready(ready, k);
         if (__any_sync(0xffffffffu, amax > 0.0)) amax = warp_max(amax);
-        const double ap = fabs(piv);
         if (!(ap > 0.0) || !isfinite(piv)) {
             bad |= ST_SINGULAR;
             // The first singular column: a minimum (spread mode: the sync
