@@ -354,7 +354,10 @@ lu_factor_par_kernel(int n, const int* Ap, const int* Ai, const double* Ax, cons
         if (lane == 0) {
             s_beg = -1;
             s_status = status;
-            if (status == -1) Up[n] = (int)unz;
+            if (status == -1) {     // n = 0: written here alone
+                Lp[n] = (int)lnz;
+                Up[n] = (int)unz;
+            }
         }
         __syncthreads();
         unz = __shfl_sync(0xffffffffu, unz, 0);
