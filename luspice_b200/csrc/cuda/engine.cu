@@ -604,6 +604,8 @@ void make_dense_plan(const std::vector<PatternObj*>& pats, int threads, SmemPlan
     };
     plan.dstg = dneed(3) <= budget ? 3 : 1;
     plan.bytes = dneed(plan.dstg);
+    // The inverses of the diagonal blocks: [32][34] fp64 per warp, in the same memory.
+    plan.dinv = std::min(threads / 32, (int)((plan.bytes - fixed) / (32 * 34 * sizeof(double))));
 }
 
 // CTA size of the dense-block kernel when a lone CTA takes a system: a

@@ -18,7 +18,6 @@ namespace lusp {
 struct PatternDev {
     int n, nnz_a, cap, max_col, nslices, sell_total;
     int nnz_l, nnz_u;        // strict L and strict U entries (by rows)
-    int nnz_lcol;            // strict L entries of the columns before the dense block
     int nfwd_levels, nbwd_levels;    // sweep steps (descriptors) of each sweep
     const int* cp;           // [n+1] merged column pointers
     const int* ri;           // [cap] row positions, ascending per column
@@ -42,7 +41,7 @@ struct PatternDev {
     const int* sell_perm;    // [32*nslices] row position or -1
     const int* rowat;        // [n] position -> original row
     const int* q;            // [n] position -> original column
-    const int* lp;           // [n+1] packed strict-L columns (SysDev::lcol)
+    const int* lp;           // [n+1] packed strict-L columns (packed_l)
     const int4* seg;         // update segments (StaticPattern::seg; null: search rows)
     const unsigned short* rel;    // ... and their relative slots
     // Dense trailing block: rows/columns [k0, n), dtail = n - k0 (0: none);
@@ -64,6 +63,7 @@ struct PatternDev {
     const int* fwd_ldesc;    // [nfwd_levels * 5] level descriptors (see host)
     const int* bwd_ldesc;    // [nbwd_levels * 5]
     int lev_max_ent, lev_max_rows;   // widest sweep level (entries, rows)
+    int nnz_lcol;            // strict L entries of the columns before the dense block
 };
 
 // Per-system statistics written by the kernels.
@@ -93,12 +93,15 @@ struct SysStats {
     long long cyc_tdiag, cyc_tgemv;
 };
 
-// One system: pattern + values + vectors + workspace.
+// One system: pattern + values + vectors + workspace.  The solve kernels hold
+// a copy in registers, and where a field of this struct, of PatternDev or of
+// SmemPlan lies is enough to move their register assignment (12 bytes more
+// spilled: solves 0.9-1.2 % slower), so fields that the solves do not read
+// stay behind or out of them.
 struct SysDev {
     const PatternDev* pat;
     const double* a_val;     // [nnz_a] input values, fp64
     void* lu;                // [cap] merged factor values (VT)
-    void* lcol;              // [nnz_lcol] packed strict L columns before the dense block (VT)
     void* lval;              // [nnz_l] strict L by rows (VT)
     void* uval;              // [nnz_u] strict U by rows (VT)
     void* udiag;             // [n] U(k,k) (VT)
@@ -110,7 +113,8 @@ struct SysDev {
     double* cs;              // [n] Ruiz column scaling
     const double* b;         // [n] right-hand side, original row order
     double* x;               // [n] solution, original column order
-    double* work;            // workspace (see solve phase)
+    double* work;            // workspace of the refactorization (packed strict
+                             // L, see packed_l) and of the solve phase
     double* scratch;         // per-CTA refactor spill (columns longer than
                              // the shared-memory work area), may be null
     void* tail;              // [dtail * tail_ld] dense L\U of the trailing
@@ -165,9 +169,24 @@ __host__ __device__ inline size_t tinv_bytes(const SysSizes& z, size_t vs) {
     return ((z.dtail + 31) / 32) * 2048 * vs;
 }
 
+// Workspace of one system: the packed strict L is read by the refactorization
+// alone and the Krylov vectors are written and read by the solve alone, so
+// both use the same memory.  With the default krylov the vectors are the
+// larger (a copy of its own would make the n = 4050 grid's system 10 % larger
+// in mixed precision and 14 % in fp64).
+__host__ __device__ inline size_t work_bytes(const SysSizes& z, size_t vs, int m) {
+    const size_t vectors = (2 * (size_t)m + 8) * z.n * 8, lcol = z.nnz_lcol * vs;
+    return vectors > lcol ? vectors : lcol;
+}
+
+// Packed strict L columns before the dense block, [nnz_lcol] VT: valid while
+// the refactorization runs.
+template <typename VT>
+__device__ inline VT* packed_l(const SysDev& S) { return (VT*)S.work; }
+
 __host__ __device__ inline size_t sys_private_bytes(const SysSizes& z, size_t vs, int m) {
-    return al256(z.cap * vs + 64) + al256(z.nnz_lcol * vs + 64) + al256(z.nnz_l * vs + 64) + al256(z.nnz_u * vs + 64) + al256(z.n * vs) +
-           al256(z.n * vs + 64) + al256(z.sell * 8) + al256(z.sell * 4) + al256((2 * (size_t)m + 8) * z.n * 8) +
+    return al256(z.cap * vs + 64) + al256(z.nnz_l * vs + 64) + al256(z.nnz_u * vs + 64) + al256(z.n * vs) +
+           al256(z.n * vs + 64) + al256(z.sell * 8) + al256(z.sell * 4) + al256(work_bytes(z, vs, m)) +
            al256(z.dtail * z.tail_ld * vs) + al256(z.dtail * z.tail_ld * 8) + al256(z.sell * 2) +
            2 * al256(z.n * 8) + al256(tinv_bytes(z, vs));
 }
@@ -180,14 +199,13 @@ __host__ __device__ inline char* sys_carve(SysDev& D, char* p, const SysSizes& z
     D.tailw = z.dtail > 0 ? (double*)p : nullptr;
     p += al256(z.dtail * z.tail_ld * 8);
     D.lu = p; p += al256(z.cap * vs + 64);
-    D.lcol = p; p += al256(z.nnz_lcol * vs + 64);
     D.lval = p; p += al256(z.nnz_l * vs + 64);
     D.uval = p; p += al256(z.nnz_u * vs + 64);
     D.udiag = p; p += al256(z.n * vs);
     D.udiag_bwd = p; p += al256(z.n * vs + 64);
     D.sell64 = (double*)p; p += al256(z.sell * 8);
     D.sell32 = (float*)p; p += al256(z.sell * 4);
-    D.work = (double*)p; p += al256((2 * (size_t)m + 8) * z.n * 8);
+    D.work = (double*)p; p += al256(work_bytes(z, vs, m));
     D.sell16 = p; p += al256(z.sell * 2);
     D.rs = (double*)p; p += al256(z.n * 8);
     D.cs = (double*)p; p += al256(z.n * 8);
@@ -240,6 +258,7 @@ struct SmemPlan {
     int wcap;                // per-warp refactor work slots
     int drows;               // dense trailing block: rows of a block column
     int dstg;                // ... and panel row groups in flight per warp (1 or 3)
+    int dinv;                // ... and warps that invert its diagonal blocks
     int sc_ent, sc_rows;     // sweep stage capacity (entries, rows; 0: no stages)
     int ycap;                // doubles for a shared-memory solve vector
     int dcap;                // ints for shared-memory sweep descriptors
