@@ -608,11 +608,20 @@ void make_dense_plan(const std::vector<PatternObj*>& pats, int threads, SmemPlan
     plan.dinv = std::min(threads / 32, (int)((plan.bytes - fixed) / (32 * 34 * sizeof(double))));
 }
 
-// CTA size of the dense-block kernel when a lone CTA takes a system: a
-// thread per row of the block, up to 512, so that small blocks share an SM
-// (768 circuits with D up to 128, B200: four CTAs of 128 threads per SM
-// 0.27 ms; the block's chain, not its arithmetic, fills a CTA's time).
-static int dense_block_threads(int dmax) { return dmax <= 128 ? 128 : dmax <= 256 ? 256 : 512; }
+// CTA size of the dense-block kernel when a lone CTA takes a system.  A CTA's
+// time is the chain of the block's panels, shortened by more updating warps;
+// smaller CTAs let several share an SM, which pays once a launch has more
+// systems than SMs.  So: 512 threads while every system has an SM, then a
+// thread per row of the block where that many CTAs are needed, 256 for two
+// systems per SM.  B200, us per launch with 128 / 256 / 512 threads:
+//   D =  96: 148 systems 129 / 105 / 100, 296: 145 / 125 / 203, 600: 299 / 336 / 487
+//   D = 128: 148 systems 207 / 166 / 147, 296: 234 / 198 / 302, 600: 473 / 541 / 727
+//   D = 256: 148 systems 1005 / 584 / 477, 296: 1072 / 683 / 939, 600: 3093 / 1868 / 2310
+//   D = 400: one CTA per SM of any size, 600 systems 17295 / 9050 / 6114
+static int dense_block_threads(int dmax, int nsys) {
+    if (nsys <= sm_count() || dmax > 256) return 512;
+    return dmax <= 128 && nsys > 2 * sm_count() ? 128 : 256;
+}
 
 // Raise the dynamic shared-memory limit of one kernel (once per size; not a
 // stream operation, so it stays out of captured graphs after the first
@@ -1089,7 +1098,7 @@ int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& 
         if (a.dcluster == 1) {
             int dmax = 0, docc = 0;
             for (auto* p : pats) dmax = std::max(dmax, p->S.dtail);
-            a.dblock = dense_block_threads(dmax);
+            a.dblock = dense_block_threads(dmax, ntail);
             make_dense_plan(pats, a.dblock, a.dplan);
             rc = o.prec == LUSP_FP64 ? dense_prepare<double>(a.dplan.bytes, a.dblock, &docc)
                                      : dense_prepare<float>(a.dplan.bytes, a.dblock, &docc);
