@@ -981,9 +981,17 @@ void fill_params(SolveParams& prm, const lusp_batch_opts& o) {
 // has 5.9 M).
 constexpr long long kSpreadMinUpdates = 16ll << 20;
 // Gathered updates per system above which a batch of at most one system
-// per SM spreads each system over up to kSpreadMidGroup 256-thread CTAs.
+// per SM spreads each system over up to kSpreadMidGroup 256-thread CTAs,
+// when that gives a system at least kSpreadMidLeast of them; with fewer, one
+// 768-thread CTA per system is faster.  B200, us (mixed / fp64), spread
+// against one CTA: 80 systems (7 CTAs each) n = 5000 circuit 825 / 947
+// against 1054 / 1188, n = 2000 grid 682 / 769 against 691 / 792; 90 systems
+// (6) 936 / 1080 against 1056 / 1192 and 724 / 819 against 693 / 792; 100
+// systems (5) 1090 / 1251 against 1059 / 1198 and 800 / 895 against 694 / 794;
+// 148 systems (4) 1354 / 1576 against 1111 / 1233 and 938 / 1051 against
+// 710 / 811.
 constexpr long long kSpreadMidUpdates = 1ll << 17;
-constexpr int kSpreadMidGroup = 12;
+constexpr int kSpreadMidGroup = 12, kSpreadMidLeast = 6;
 
 int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& o, int nsys, LaunchArgs& a) {
     a.rblock = refactor_block(o, nsys);
@@ -1038,7 +1046,7 @@ int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& 
             rc = refactor_occupancy(o.prec, pl.bytes, 256, &mocc, true);
             if (rc != LUSP_OK) return rc;
             const int mg = std::min(kSpreadMidGroup, mocc * sm_count() / nsys);
-            if (mg >= 4) {
+            if (mg >= kSpreadMidLeast) {
                 g = mg;
                 mid = true;
                 a.rblock = 256;
