@@ -20,9 +20,13 @@
 // barrier), the next column's input and the next dependency's pointers loaded
 // ahead; the other warps join only for an update of more than kLongColumn
 // rows.  The row permutation is kept in shared memory (16 bits: n is below
-// 19,400 there).  n = 989 circuit, B200, factor and solve: 8.15 -> 5.48 ms
-// against a CTA-wide scan of all n rows per column (factor 4.92, solve 0.55
-// ms; a lane walking its word of the bitmap instead of the list: 6.85 ms).
+// 19,400 there).  B200, factor in ms against a CTA-wide scan of all n rows per
+// column and a CTA-wide step per dependency: n = 989 circuit 7.26 -> 4.88 (a
+// lane walking its word of the bitmap instead of the list: 6.85), n = 4050 grid
+// 116 -> 79, dense n = 600 221 -> 192, band matrix n = 2000 with 120 diagonals
+// on each side 303 -> 265.  The input's entries go in 32 at a time, in order: a
+// lane looking for later duplicates of its entry took half the time of a dense
+// matrix (n = 600: 410 ms).
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -32,8 +36,13 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// Rows of an update above which all warps share it.
-constexpr int kLongColumn = 256;
+// Rows of an update above which all warps share it: what one warp does in one
+// step.  B200, factor in ms with 16 / 24 / 32 / 40 / 48 / 64: the n = 4050 grid
+// (L columns of up to 146 rows) 80.0 / 79.6 / 79.4 / 80.4 / 81.7 / 84.1, band
+// matrix n = 2000 with 60 diagonals on each side 119 / 119 / 119 / 119 / 119 /
+// 133, an n = 4000 circuit with supply nets 71.9 / 71.8 / 71.7 / 72.4 / 79.4 /
+// 82.7 (a CTA-wide step for every update: 117, 141, 108).
+constexpr int kLongColumn = 32;
 constexpr unsigned short kNone = 0xffffu;
 
 // Inclusive prefix sum over a warp.
@@ -119,32 +128,27 @@ lu_factor_par_kernel(int n, const int* Ap, const int* Ai, const double* Ax, cons
                 Lp[k] = (int)lnz;
                 Up[k] = (int)unz;
             }
-            // 1. x = A(:,k) (assignment, the last duplicate wins) and seeds,
-            //    the first 32 entries loaded a column ahead.
+            // 1. x = A(:,k) (assignment, the last duplicate wins) and seeds, 32
+            //    entries at a time in order, the first of them loaded a column
+            //    ahead: of equal rows in a group the last lane stores, and a
+            //    later group stores over an earlier one.
             const int a0 = na0, a1 = na1, ck = nck, mi = ni;
             const double mx = nx;
             fetch(k + 1);
-            {
-                const bool in = a0 + lane < a1;
-                const unsigned same = __match_any_sync(0xffffffffu, in ? mi : -1 - lane);
-                bool last = in && (same >> lane) == 1u;
-                for (int p = a0 + 32; p < a1 && last; p++) last = Ai[p] != mi;
-                if (last) x[mi] = mx;
-                if (in) {
-                    atomicOr(touched + (mi >> 5), 1u << (mi & 31));
-                    const int J = pos[mi];
+            auto seed = [&](int i, double v) {      // i < 0: no entry
+                const unsigned same = __match_any_sync(0xffffffffu, i);
+                if (i >= 0) {
+                    if ((same >> lane) == 1u) x[i] = v;
+                    atomicOr(touched + (i >> 5), 1u << (i & 31));
+                    const int J = pos[i];
                     if (J != kNone) atomicOr(cand + (J >> 5), 1u << (J & 31));
                 }
-            }
-            for (int p = a0 + 32 + lane; p < a1; p += 32) {
-                const int i = Ai[p];
-                bool last = true;
-                for (int p2 = p + 1; p2 < a1; p2++)
-                    if (Ai[p2] == i) { last = false; break; }
-                if (last) x[i] = Ax[p];
-                atomicOr(touched + (i >> 5), 1u << (i & 31));
-                const int J = pos[i];
-                if (J != kNone) atomicOr(cand + (J >> 5), 1u << (J & 31));
+            };
+            seed(mi, mx);
+            for (int p = a0 + 32; p < a1; p += 32) {
+                __syncwarp();
+                const bool in = p + lane < a1;
+                seed(in ? Ai[p + lane] : -1, in ? Ax[p + lane] : 0.0);
             }
             __syncwarp();
             // 2. Left-looking updates in ascending pivot position; the
@@ -161,11 +165,11 @@ lu_factor_par_kernel(int n, const int* Ap, const int* Ai, const double* Ax, cons
                     const unsigned wb = __shfl_sync(0xffffffffu, bits, src);
                     const int j = ((w0 + src) << 5) + (__ffs(wb) - 1);
                     if (j != pj) {
-                        pp0 = Lp[j] + 1;
+                        pp0 = Lp[j];
                         pp1 = Lp[j + 1];
                         prow = rowat[j];
                     }
-                    const int p0 = pp0, p1 = pp1;
+                    const int p0 = pp0 + 1, p1 = pp1;
                     const double xr = x[prow];
                     // The next set bit: in this word or the next non-empty one.
                     const unsigned rest = wb & (wb - 1u), more = any & (any - 1u);
@@ -174,7 +178,7 @@ lu_factor_par_kernel(int n, const int* Ap, const int* Ai, const double* Ax, cons
                     pj = rest ? ((w0 + src) << 5) + (__ffs(rest) - 1)
                               : nsrc >= 0 ? ((w0 + nsrc) << 5) + (__ffs(nb) - 1) : -1;
                     if (pj >= 0) {
-                        pp0 = Lp[pj] + 1;
+                        pp0 = Lp[pj];
                         pp1 = Lp[pj + 1];
                         prow = rowat[pj];
                     }
