@@ -392,10 +392,10 @@ lu_factor_par_kernel(int n, const int* Ap, const int* Ai, const double* Ax, cons
 // columns from the last down, v[k] = v[k] / diagonal (the column's last entry);
 // else from the first up (the first entry), in both v[i] -= entry * v[k] for
 // the column's other entries, separately rounded.  The pointers of 32 columns
-// are loaded together, a column's first 32 entries and its diagonal four
-// columns ahead, so the chain of a column is the shared-memory round trip of v
-// and the update.
-template <bool UPPER>
+// are loaded together, the diagonal and the first 32 CH entries of a column
+// AHEAD columns ahead, so the chain of a column is the shared-memory round trip
+// of v and the update; longer columns load 128 entries at a time.
+template <bool UPPER, int CH, int AHEAD>
 __device__ void trisolve_sweep(int n, const int* cp, const int* ci, const double* cx, double* v) {
     const int lane = threadIdx.x & 31;
     int pb = 0, pe = 0;                     // pointers of column (32 block + lane) in sweep order
@@ -410,25 +410,26 @@ __device__ void trisolve_sweep(int n, const int* cp, const int* ci, const double
         p0 = __shfl_sync(0xffffffffu, pb, t & 31);
         p1 = __shfl_sync(0xffffffffu, pe, t & 31);
     };
-    // Entries beside the diagonal: [p0 + 1, p1) of L, [p0, p1 - 1) of U, of
-    // the next kAhead columns.
-    constexpr int kAhead = 4;
-    int p0[kAhead], p1[kAhead], i[kAhead];
-    double e[kAhead], dg[kAhead];
+    // Entries beside the diagonal: [p0 + 1, p1) of L, [p0, p1 - 1) of U.
+    int p0[AHEAD], p1[AHEAD], i[AHEAD][CH];
+    double e[AHEAD][CH], dg[AHEAD];
     auto fetch = [&](int t, int u) {
         bounds(t, p0[u], p1[u]);
         const int q = UPPER ? p0[u] + lane : p0[u] + 1 + lane, end = UPPER ? p1[u] - 1 : p1[u];
-        i[u] = q < end ? ci[q] : -1;
-        e[u] = q < end ? cx[q] : 0.0;
+#pragma unroll
+        for (int c = 0; c < CH; c++) {
+            i[u][c] = q + 32 * c < end ? ci[q + 32 * c] : -1;
+            e[u][c] = q + 32 * c < end ? cx[q + 32 * c] : 0.0;
+        }
         dg[u] = cx[UPPER ? p1[u] - 1 : p0[u]];
     };
 #pragma unroll
-    for (int u = 0; u < kAhead; u++)
+    for (int u = 0; u < AHEAD; u++)
         if (u < n) fetch(u, u);
     double rd = n > 0 ? __drcp_rn(dg[0]) : 1.0;
-    for (int t0 = 0; t0 < n; t0 += kAhead) {
+    for (int t0 = 0; t0 < n; t0 += AHEAD) {
 #pragma unroll
-        for (int u = 0; u < kAhead; u++) {
+        for (int u = 0; u < AHEAD; u++) {
             const int t = t0 + u;
             if (t >= n) break;
             const int k = UPPER ? n - 1 - t : t;
@@ -436,21 +437,83 @@ __device__ void trisolve_sweep(int n, const int* cp, const int* ci, const double
             const double vk = d == 1.0 ? v[k] : lusp::div_by<false>(v[k], d, r);
             __syncwarp();
             if (lane == 0) v[k] = vk;
-            if (i[u] >= 0) v[i[u]] = __dsub_rn(v[i[u]], __dmul_rn(e[u], vk));
+#pragma unroll
+            for (int c = 0; c < CH; c++)
+                if (i[u][c] >= 0) v[i[u][c]] = __dsub_rn(v[i[u][c]], __dmul_rn(e[u][c], vk));
             const int end = UPPER ? p1[u] - 1 : p1[u];
-            for (int q = (UPPER ? p0[u] : p0[u] + 1) + 32 + lane; q < end; q += 32) {
-                const int i2 = ci[q];
-                v[i2] = __dsub_rn(v[i2], __dmul_rn(cx[q], vk));
+            for (int q = (UPPER ? p0[u] : p0[u] + 1) + 32 * CH + lane; q - lane < end; q += 128) {
+                int i4[4];
+                double e4[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    i4[c] = q + 32 * c < end ? ci[q + 32 * c] : -1;
+                    e4[c] = q + 32 * c < end ? cx[q + 32 * c] : 0.0;
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (i4[c] >= 0) v[i4[c]] = __dsub_rn(v[i4[c]], __dmul_rn(e4[c], vk));
             }
-            if (t + kAhead < n) fetch(t + kAhead, u);
-            if (t + 1 < n && dg[(u + 1) % kAhead] != 1.0) rd = __drcp_rn(dg[(u + 1) % kAhead]);
+            if (t + AHEAD < n) fetch(t + AHEAD, u);
+            if (t + 1 < n && dg[(u + 1) % AHEAD] != 1.0) rd = __drcp_rn(dg[(u + 1) % AHEAD]);
             __syncwarp();
         }
     }
 }
 
-// Systems whose solve vector fits the kernel's static shared memory.
+// The same sweep by the whole CTA for a vector in global memory: out[k] =
+// in[k] / diagonal, in[i] -= entry * out[k].  A thread's first entry of the
+// next column is loaded before the barrier that ends this one, the pointers a
+// column earlier: n = 8000 grid 8320 -> 7470 us (B200; without the early loads
+// 9120 beside the static shared memory of the small systems, which leaves less
+// L1 for the vectors).
+template <bool UPPER>
+__device__ void trisolve_sweep_cta(int n, const int* cp, const int* ci, const double* cx, double* in, double* out) {
+    const int tid = threadIdx.x, nt = blockDim.x;
+    auto column = [&](int t) { return UPPER ? n - 1 - t : t; };
+    int b0 = 0, b1 = 0, ni = -1;            // the next column: pointers, this thread's entry, diagonal
+    double ne = 0.0, nd = 1.0;
+    auto fetch = [&]() {
+        const int q = UPPER ? b0 + tid : b0 + 1 + tid, end = UPPER ? b1 - 1 : b1;
+        ni = q < end ? ci[q] : -1;
+        ne = q < end ? cx[q] : 0.0;
+        nd = cx[UPPER ? b1 - 1 : b0];
+    };
+    auto pointers = [&](int t, int& q0, int& q1) {
+        q0 = cp[column(t)];
+        q1 = cp[column(t) + 1];
+    };
+    int f0 = 0, f1 = 0;
+    if (n > 0) pointers(0, b0, b1);
+    if (n > 0) fetch();
+    if (n > 1) pointers(1, f0, f1);
+    for (int t = 0; t < n; t++) {
+        const int k = column(t), p0 = b0, p1 = b1, i = ni;
+        const double e = ne, d = nd, vk = d == 1.0 ? in[k] : __ddiv_rn(in[k], d);
+        b0 = f0;
+        b1 = f1;
+        if (t + 1 < n) fetch();
+        if (t + 2 < n) pointers(t + 2, f0, f1);
+        if (tid == 0) out[k] = vk;
+        if (i >= 0) in[i] = __dsub_rn(in[i], __dmul_rn(e, vk));
+        const int end = UPPER ? p1 - 1 : p1;
+        for (int q = (UPPER ? p0 : p0 + 1) + nt + tid; q < end; q += nt) {
+            const int j = ci[q];
+            in[j] = __dsub_rn(in[j], __dmul_rn(cx[q], vk));
+        }
+        __syncthreads();
+    }
+}
+
+// Systems whose solve vector fits the kernel's static shared memory.  B200,
+// us a solve against the whole CTA on a vector in global memory: n = 989 circuit
+// 872 -> 514, n = 4050 grid 3961 -> 2713, dense n = 600 1429 -> 1265.
 constexpr int kTriShared = 6000;
+// Mean entries per column of L or U above which a sweep loads 128 entries of a
+// column two columns ahead, else 32 entries four columns ahead.  B200, us a
+// solve with 32 / 128: band matrices n = 2000 with 60 diagonals on each side
+// 2285 / 1621, with 120 2980 / 2283, dense n = 200 248 / 217; n = 989 circuit
+// (7 entries) 514 / 749, n = 4050 grid (28) 2712 / 3230.
+constexpr int kTriLong = 48;
 
 // pb = P b; L y = pb by columns (unit diagonal first); U z = y by columns
 // (diagonal last); x = Q z.  Same operation sequence as splu.h:210-239, so
@@ -466,41 +529,32 @@ trisolve_par_kernel(int n, const int* Lp, const int* Li, const double* Lx, const
     __shared__ double sv[kTriShared];
     const int tid = threadIdx.x, nt = blockDim.x;
     int* rowat = work_i;
-    double* pb = n <= kTriShared ? sv : work_d;
-    double* y = work_d + n;
     for (int i = tid; i < n; i += nt) rowat[i] = -1;
     __syncthreads();
     for (int i = tid; i < n; i += nt)
         if (pinv[i] >= 0) rowat[pinv[i]] = i;
     __syncthreads();
-    for (int k = tid; k < n; k += nt) pb[k] = rowat[k] >= 0 ? b[rowat[k]] : 0.0;
-    __syncthreads();
     if (n <= kTriShared) {
-        if (tid < 32) {
-            trisolve_sweep<false>(n, Lp, Li, Lx, sv);
-            trisolve_sweep<true>(n, Up, Ui, Ux, sv);
+        for (int k = tid; k < n; k += nt) sv[k] = rowat[k] >= 0 ? b[rowat[k]] : 0.0;
+        __syncthreads();
+        if (tid < 32 && n > 0) {
+            if (Lp[n] <= (long)kTriLong * n) trisolve_sweep<false, 1, 4>(n, Lp, Li, Lx, sv);
+            else trisolve_sweep<false, 4, 2>(n, Lp, Li, Lx, sv);
+            if (Up[n] <= (long)kTriLong * n) trisolve_sweep<true, 1, 4>(n, Up, Ui, Ux, sv);
+            else trisolve_sweep<true, 4, 2>(n, Up, Ui, Ux, sv);
         }
         __syncthreads();
         for (int k = tid; k < n; k += nt) x[q ? q[k] : k] = sv[k];
         return;
     }
-    for (int k = 0; k < n; k++) {
-        const double yk = __ddiv_rn(pb[k], Lx[Lp[k]]);
-        if (tid == 0) y[k] = yk;
-        for (int p = Lp[k] + 1 + tid; p < Lp[k + 1]; p += nt)
-            pb[Li[p]] = __dsub_rn(pb[Li[p]], __dmul_rn(Lx[p], yk));
-        __syncthreads();
-    }
+    double* pb = work_d;
+    double* y = work_d + n;
+    for (int k = tid; k < n; k += nt) pb[k] = rowat[k] >= 0 ? b[rowat[k]] : 0.0;
+    __syncthreads();
+    trisolve_sweep_cta<false>(n, Lp, Li, Lx, pb, y);
     // z overwrites pb (no longer needed).
-    double* z = pb;
-    for (int k = n - 1; k >= 0; k--) {
-        const double zk = __ddiv_rn(y[k], Ux[Up[k + 1] - 1]);
-        if (tid == 0) z[k] = zk;
-        for (int p = Up[k] + tid; p < Up[k + 1] - 1; p += nt)
-            y[Ui[p]] = __dsub_rn(y[Ui[p]], __dmul_rn(Ux[p], zk));
-        __syncthreads();
-    }
-    for (int k = tid; k < n; k += nt) x[q ? q[k] : k] = z[k];
+    trisolve_sweep_cta<true>(n, Up, Ui, Ux, y, pb);
+    for (int k = tid; k < n; k += nt) x[q ? q[k] : k] = pb[k];
 }
 
 extern "C" int lusp_lu_factor_par_launch(int n, const int* Ap, const int* Ai, const double* Ax,
