@@ -65,48 +65,51 @@ template <> __device__ __forceinline__ double ldv<__half>(const __half* p) {
 }
 
 // Blocks [0, sell_blocks) take the slices, a warp each; the blocks after them
-// take the long rows, a block per row (fixed-order reduction): a supply net's
-// row of 800 entries is then one round of loads, where a warp walking it
-// (seven rounds of four loads a lane) was the whole launch.  n = 40,000 circuit
-// with four such rows, fp32, B200: 8.2 -> 6.1 us a product.
-// WIDE (all warps resident at once, so a warp's latency is the launch's): row
-// numbers and up to eight entries per lane requested before the first is
-// used: 6.1 -> 4.1 us there.  Larger matrices stream (a mesh of 2 M nodes, fp64,
-// at 4.1 TB/s) and are 0.8 % slower that way (two or four slices per warp: 11 %).
-template <int C, bool WIDE, typename VT>
-__global__ void __launch_bounds__(256)
+// take the long rows, LW warps per row (8: a block, or 1), lanes over its
+// entries with four partial sums, fixed-order reductions.  WIDE: row numbers
+// and up to eight entries per lane requested before the first is used; the
+// other instances have no bound on resident blocks (one changes the order of
+// their loads: a mesh of 1 M nodes 12.0 -> 16.1 us).  Which of them a product
+// takes, and why, is said at sell_value.
+constexpr int kWideBlocks = 4;      // resident blocks per SM of the wide instances
+template <int C, bool WIDE, int LW, typename VT>
+__global__ void __launch_bounds__(256, WIDE ? kWideBlocks : 0)
 sell_kernel(int nslices, const int* __restrict__ ptr, const int* __restrict__ col,
             const VT* __restrict__ val, const int* __restrict__ perm,
             const double* __restrict__ x, double* __restrict__ y,
-            const double* __restrict__ row_div, int sell_blocks,
+            const double* __restrict__ row_div, int sell_blocks, int nlong,
             const int* __restrict__ lrow, const int* __restrict__ lptr, const int* __restrict__ lcol,
             const VT* __restrict__ lval) {
     if ((int)blockIdx.x >= sell_blocks) {
+        constexpr int T = 32 * LW;                                      // threads of a row
         __shared__ double part[8];
-        const int w = (int)blockIdx.x - sell_blocks;
+        const int w = (((int)blockIdx.x - sell_blocks) * 256 + (int)threadIdx.x) / T;
+        if (w >= nlong) return;                                         // LW = 1: a whole warp
         const int p1 = lptr[w + 1];
         double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-        int p = lptr[w] + (int)threadIdx.x;
-        for (; p + 768 < p1; p += 1024) {
-            const int c0 = lcol[p], c1 = lcol[p + 256], c2 = lcol[p + 512], c3 = lcol[p + 768];
+        int p = lptr[w] + (int)threadIdx.x % T;
+        for (; p + 3 * T < p1; p += 4 * T) {
+            const int c0 = lcol[p], c1 = lcol[p + T], c2 = lcol[p + 2 * T], c3 = lcol[p + 3 * T];
             a0 = fma(ldv<VT>(lval + p), __ldg(x + c0), a0);
-            a1 = fma(ldv<VT>(lval + p + 256), __ldg(x + c1), a1);
-            a2 = fma(ldv<VT>(lval + p + 512), __ldg(x + c2), a2);
-            a3 = fma(ldv<VT>(lval + p + 768), __ldg(x + c3), a3);
+            a1 = fma(ldv<VT>(lval + p + T), __ldg(x + c1), a1);
+            a2 = fma(ldv<VT>(lval + p + 2 * T), __ldg(x + c2), a2);
+            a3 = fma(ldv<VT>(lval + p + 3 * T), __ldg(x + c3), a3);
         }
         // At most three entries per thread are left.
-        const bool b0 = p < p1, b1 = p + 256 < p1, b2 = p + 512 < p1;
-        const int c0 = b0 ? lcol[p] : 0, c1 = b1 ? lcol[p + 256] : 0, c2 = b2 ? lcol[p + 512] : 0;
+        const bool b0 = p < p1, b1 = p + T < p1, b2 = p + 2 * T < p1;
+        const int c0 = b0 ? lcol[p] : 0, c1 = b1 ? lcol[p + T] : 0, c2 = b2 ? lcol[p + 2 * T] : 0;
         if (b0) a0 = fma(ldv<VT>(lval + p), __ldg(x + c0), a0);
-        if (b1) a1 = fma(ldv<VT>(lval + p + 256), __ldg(x + c1), a1);
-        if (b2) a2 = fma(ldv<VT>(lval + p + 512), __ldg(x + c2), a2);
+        if (b1) a1 = fma(ldv<VT>(lval + p + T), __ldg(x + c1), a1);
+        if (b2) a2 = fma(ldv<VT>(lval + p + 2 * T), __ldg(x + c2), a2);
         double acc = (a0 + a1) + (a2 + a3);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
+        if (LW > 1) {
+            if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+            __syncthreads();
             acc = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
+        }
+        if (threadIdx.x % T == 0) {
             const int row = lrow[w];
             y[row] = row_div ? acc / row_div[row] : acc;
         }
@@ -196,33 +199,55 @@ struct SellObj {
     double* d_xs = nullptr;     // fp16: scaled x
     double smin = 0, smax = 0;
     // Rows much longer than the rest (supply nets) stay out of the slices
-    // (one of them would set a whole slice's width): CSR, a block per row.
+    // (one of them would set a whole slice's width): CSR.
     int nlong = 0;
+    long long_stored = 0;       // entries of the long rows
     int* d_lrow = nullptr;      // [nlong] row
     int* d_lptr = nullptr;      // [nlong+1]
     int* d_lcol = nullptr;
     void* d_lval = nullptr;
 };
 
-template <int C, typename VT>
-static void sell_value(const SellObj* S, int grid, int sell_blocks, bool wide, const double* x, double* y,
-                       const double* rsc, cudaStream_t st) {
-    if (wide)
-        sell_kernel<C, true, VT><<<grid, 256, 0, st>>>(S->nslices, S->d_ptr, S->d_col, (const VT*)S->d_val, S->d_perm, x, y,
-                                                      rsc, sell_blocks, S->d_lrow, S->d_lptr, S->d_lcol,
-                                                      (const VT*)S->d_lval);
-    else
-        sell_kernel<C, false, VT><<<grid, 256, 0, st>>>(S->nslices, S->d_ptr, S->d_col, (const VT*)S->d_val, S->d_perm, x, y,
-                                                       rsc, sell_blocks, S->d_lrow, S->d_lptr, S->d_lcol,
+template <int C, bool WIDE, int LW, typename VT>
+static void sell_launch(const SellObj* S, int grid, int sell_blocks, const double* x, double* y, const double* rsc,
+                        cudaStream_t st) {
+    sell_kernel<C, WIDE, LW, VT><<<grid, 256, 0, st>>>(S->nslices, S->d_ptr, S->d_col, (const VT*)S->d_val, S->d_perm, x,
+                                                       y, rsc, sell_blocks, S->nlong, S->d_lrow, S->d_lptr, S->d_lcol,
                                                        (const VT*)S->d_lval);
 }
 
+// The product's kernel (see sell_kernel).  B200, replayed graphs of 50 products
+// of fp64 values, us.
+//   Long rows: a block each while their blocks are resident at once (8 per SM)
+//   or from 768 entries on, else a warp each, which shares the reduction's cost
+//   among fewer lanes: 40,000 short rows with 100 rows of 300 entries 2.6 / 3.8
+//   (block / warp), 1000 4.2 / 4.1, 2000 6.2 / 5.1, 4000 9.7 / 7.7, with 3000
+//   of 700 11.8 / 10.4, 2000 of 1000 11.1 / 17.8.
+//   Wide slices while every block is resident, so that a warp's latency is the
+//   launch's: a mesh of 20,000 nodes 1.98 / 2.64 (wide / not), of 151,000
+//   (4705 slices) 2.80 / 3.21; of 153,000 (4778) 3.44 / 3.25, of 1 M
+//   13.6 / 12.0.  A long row's block counts: 140,000 short rows with 40 long
+//   ones 3.3 / 3.7, with 100 4.1 / 3.7.  And for very long rows that are most of
+//   the product, whose loads the 64 registers of the wide instances hold:
+//   60,000 short rows with 800 of 10,000 entries 19.8 / 25.0, with 444 of 3000
+//   7.8 / 7.7.
+template <int C, typename VT>
+static void sell_value(const SellObj* S, const double* x, double* y, const double* rsc, cudaStream_t st) {
+    const int sms = lusp::sm_count(), sell_blocks = (int)(((long)S->nslices * 32 + 255) / 256);
+    const bool block = S->nlong <= 8 * sms || S->long_stored >= 768L * S->nlong;
+    const bool very = S->nlong > 0 && S->long_stored >= 4096L * S->nlong && 2 * S->long_stored >= S->stored;
+    const int grid = sell_blocks + (block ? S->nlong : (S->nlong + 7) / 8);
+    if (grid == 0) return;
+    if (!block) sell_launch<C, false, 1, VT>(S, grid, sell_blocks, x, y, rsc, st);
+    else if (grid <= kWideBlocks * sms || very) sell_launch<C, true, 8, VT>(S, grid, sell_blocks, x, y, rsc, st);
+    else sell_launch<C, false, 8, VT>(S, grid, sell_blocks, x, y, rsc, st);
+}
+
 template <int C>
-static void sell_kind(const SellObj* S, int grid, int sell_blocks, bool wide, const double* x, double* y,
-                      const double* rsc, cudaStream_t st) {
-    if (S->kind == 0) sell_value<C, double>(S, grid, sell_blocks, wide, x, y, rsc, st);
-    else if (S->kind == 1) sell_value<C, float>(S, grid, sell_blocks, wide, x, y, rsc, st);
-    else sell_value<C, __half>(S, grid, sell_blocks, wide, x, y, rsc, st);
+static void sell_kind(const SellObj* S, const double* x, double* y, const double* rsc, cudaStream_t st) {
+    if (S->kind == 0) sell_value<C, double>(S, x, y, rsc, st);
+    else if (S->kind == 1) sell_value<C, float>(S, x, y, rsc, st);
+    else sell_value<C, __half>(S, x, y, rsc, st);
 }
 
 // Ruiz equilibration (max norm): alternately scale rows and columns by
@@ -443,7 +468,8 @@ int lusp_sell_create(int n, const int* rowptr, const int* colidx, const double* 
                 }
                 lptr[t + 1] = (int)lcol.size();
             }
-            S->stored += (long)lcol.size();
+            S->long_stored = (long)lcol.size();
+            S->stored += S->long_stored;
             e = cudaMalloc((void**)&S->d_lrow, lrows.size() * sizeof(int));
             if (e == cudaSuccess) e = cudaMalloc((void**)&S->d_lptr, lptr.size() * sizeof(int));
             if (e == cudaSuccess) e = cudaMalloc((void**)&S->d_lcol, lcol.size() * sizeof(int));
@@ -511,16 +537,10 @@ int lusp_sell_spmv(const lusp_sell* hs, const double* d_x, double* d_y, void* st
         unscale_kernel<<<(S->n + 255) / 256, 256, 0, st>>>(S->n, d_x, S->d_cs, S->d_xs);
         xin = S->d_xs;
     }
-    const int sell_blocks = (int)(((long)S->nslices * 32 + 255) / 256);
-    const int grid = sell_blocks + S->nlong;   // a block per long row
     const double* rsc = S->kind == 2 ? S->d_rs : nullptr;
-    // Wide slices while every warp is resident at once (40 per SM).
-    const bool wide = S->nslices <= 40 * lusp::sm_count();
-    if (grid > 0) {
-        if (S->C == 8) sell_kind<8>(S, grid, sell_blocks, wide, xin, d_y, rsc, st);
-        else if (S->C == 16) sell_kind<16>(S, grid, sell_blocks, wide, xin, d_y, rsc, st);
-        else sell_kind<32>(S, grid, sell_blocks, wide, xin, d_y, rsc, st);
-    }
+    if (S->C == 8) sell_kind<8>(S, xin, d_y, rsc, st);
+    else if (S->C == 16) sell_kind<16>(S, xin, d_y, rsc, st);
+    else sell_kind<32>(S, xin, d_y, rsc, st);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? LUSP_OK : lusp::cuda_fail(e, "sell spmv launch");
 }
