@@ -41,7 +41,7 @@ struct PatternDev {
     const int* sell_perm;    // [32*nslices] row position or -1
     const int* rowat;        // [n] position -> original row
     const int* q;            // [n] position -> original column
-    const int* lp;           // [n+1] packed strict-L columns (packed_l)
+    const int* lp;           // [n+1] packed strict-L columns (SysDev::lcol)
     const int4* seg;         // update segments (StaticPattern::seg; null: search rows)
     const unsigned short* rel;    // ... and their relative slots
     // Dense trailing block: rows/columns [k0, n), dtail = n - k0 (0: none);
@@ -95,9 +95,10 @@ struct SysStats {
 
 // One system: pattern + values + vectors + workspace.  The solve kernels hold
 // a copy in registers, and where a field of this struct, of PatternDev or of
-// SmemPlan lies is enough to move their register assignment (12 bytes more
-// spilled: solves 0.9-1.2 % slower), so fields that the solves do not read
-// stay behind or out of them.
+// SmemPlan lies moves their register assignment (lcol among the other pointers:
+// 12 bytes more spilled, mixed solves 0.9-1.2 % slower; a count in front of
+// PatternDev's pointers: fp64 sweeps that spill, 45 %; no lcol at all: fp64
+// grids 2 %), so fields that the solves do not read stay behind.
 struct SysDev {
     const PatternDev* pat;
     const double* a_val;     // [nnz_a] input values, fp64
@@ -113,8 +114,8 @@ struct SysDev {
     double* cs;              // [n] Ruiz column scaling
     const double* b;         // [n] right-hand side, original row order
     double* x;               // [n] solution, original column order
-    double* work;            // workspace of the refactorization (packed strict
-                             // L, see packed_l) and of the solve phase
+    double* work;            // workspace of the refactorization (lcol) and of the
+                             // solve phase
     double* scratch;         // per-CTA refactor spill (columns longer than
                              // the shared-memory work area), may be null
     void* tail;              // [dtail * tail_ld] dense L\U of the trailing
@@ -126,6 +127,9 @@ struct SysDev {
                              // block's 32 x 32 diagonal blocks (VT): per block
                              // L^-1 then U^-1, element (i, c) at c * 32 + i
     SysStats* stats;
+    void* lcol;              // [nnz_lcol] packed strict L columns before the dense
+                             // block (VT), in the workspace: valid while the
+                             // refactorization runs
 };
 
 struct SolveParams {
@@ -179,11 +183,6 @@ __host__ __device__ inline size_t work_bytes(const SysSizes& z, size_t vs, int m
     return vectors > lcol ? vectors : lcol;
 }
 
-// Packed strict L columns before the dense block, [nnz_lcol] VT: valid while
-// the refactorization runs.
-template <typename VT>
-__device__ inline VT* packed_l(const SysDev& S) { return (VT*)S.work; }
-
 __host__ __device__ inline size_t sys_private_bytes(const SysSizes& z, size_t vs, int m) {
     return al256(z.cap * vs + 64) + al256(z.nnz_l * vs + 64) + al256(z.nnz_u * vs + 64) + al256(z.n * vs) +
            al256(z.n * vs + 64) + al256(z.sell * 8) + al256(z.sell * 4) + al256(work_bytes(z, vs, m)) +
@@ -205,7 +204,9 @@ __host__ __device__ inline char* sys_carve(SysDev& D, char* p, const SysSizes& z
     D.udiag_bwd = p; p += al256(z.n * vs + 64);
     D.sell64 = (double*)p; p += al256(z.sell * 8);
     D.sell32 = (float*)p; p += al256(z.sell * 4);
-    D.work = (double*)p; p += al256(work_bytes(z, vs, m));
+    D.work = (double*)p;
+    D.lcol = p;
+    p += al256(work_bytes(z, vs, m));
     D.sell16 = p; p += al256(z.sell * 2);
     D.rs = (double*)p; p += al256(z.n * 8);
     D.cs = (double*)p; p += al256(z.n * 8);

@@ -961,7 +961,7 @@ __device__ void refactor_phase(const RefactorCtx& cx, const SmemPlan& plan, char
         // complete, up to the first that is not, then the complete first part
         // of that one; it blocks only when nothing could be applied.
         const unsigned short* rel = P.rel + *(const long long*)(rec + 8);
-        const VT* lcol = packed_l<VT>(S);
+        const VT* lcol = (const VT*)S.lcol;
         for (int s0 = 0; s0 < nseg; s0 += 32) {
             if (s0 > 0) sg = s0 + lane < nseg ? __ldg(P.seg + rec[12] + s0 + lane) : make_int4(0, 0, 0, 0);
             const int ns = min(32, nseg - s0);
@@ -1098,7 +1098,7 @@ __device__ void refactor_phase(const RefactorCtx& cx, const SmemPlan& plan, char
         // not count for its ratio).
         const double ap = fabs(piv);
         double amax = 0.0;
-        VT* lk = packed_l<VT>(S) + rec[14] - d - 1;
+        VT* lk = (VT*)S.lcol + rec[14] - d - 1;
 #pragma unroll 4
         for (int t = d + 1 + lane; t < len; t += 32) {
             const double v = x[t];

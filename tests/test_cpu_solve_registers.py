@@ -3,11 +3,12 @@
 A solve kernel keeps its state in the 128 registers a thread has at 512
 threads, and what does not fit is reloaded around every sweep, product and
 reduction.  Where a descriptor or plan field lies is enough to change what
-ptxas keeps: one pointer more in SysDev and fields moved by 4 or 8 bytes raised the
-spills of the mixed kernel from 164 to 176 bytes and made solves alone 0.9 to
-1.2 % slower (B200; up to 6 % for batches of more than a system per SM in
-fp64).  This test compiles the kernels with the library's own flags and
-`-Xptxas -v` and holds the spilled bytes at the values they were tuned with.
+ptxas keeps: a pointer in the middle of SysDev and fields moved by 4 or 8
+bytes raised the spills of the mixed kernel from 164 to 176 bytes and made
+solves alone 0.9 to 1.2 % slower (B200); other places for the same fields
+leave the fp64 or the fp16 kernel's sweeps too few registers (up to 45 %).
+This test compiles the kernels with the library's own flags and `-Xptxas -v`
+and holds the spilled bytes at the values they were timed with.
 """
 import re
 import shutil
@@ -20,7 +21,7 @@ from luspice_b200 import build as b
 KERNEL = "_ZN4lusp12solve_kernel{}EEvPKNS_6SysDevEiPiNS_8SmemPlanENS_11SolveParamsEiPKi{}_NS_6EscDevEi"
 # (entry, spilled bytes): factor type and type of A in the inner products.
 LIMITS = [(KERNEL.format("Iff", "S8"), 164), (KERNEL.format("Ifd", "S8"), 164),
-          (KERNEL.format("If6__half", "S9"), 152), (KERNEL.format("Idd", "S8"), 236)]
+          (KERNEL.format("If6__half", "S9"), 180), (KERNEL.format("Idd", "S8"), 208)]
 
 
 def test_solve_kernels_spill_no_more(tmp_path):
