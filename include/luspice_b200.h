@@ -371,7 +371,7 @@ typedef struct lusp_sell lusp_sell;
  * with LUSP_EARG when a scaled value is outside the fp16 normal range).
  * Rows longer than max(256, 8 x the mean row length) are kept out of the
  * slices (one would set its whole slice's width) and computed in the same
- * launch by a block each; `stored` counts slice slots plus their entries. */
+ * launch by a block or a warp each; `stored` counts slice slots plus their entries. */
 int lusp_sell_create(int n, const int *rowptr, const int *colidx, const double *vals,
                      int C, int sigma, int value_kind, lusp_sell **out);
 void lusp_sell_destroy(lusp_sell *s);

@@ -147,8 +147,8 @@ dense_kernel(const SysDev* __restrict__ sys, int nsys, int* queue, SmemPlan plan
 }
 
 // The dense trailing blocks with a 2-CTA thread-block cluster per system
-// (the two CTAs split the trailing updates): rank 0 draws a system, both
-// read it through distributed shared memory between two cluster barriers.
+// (the CTAs take the block columns in turn): rank 0 draws a system, both read
+// it through distributed shared memory between two cluster barriers.
 template <typename VT>
 __global__ void __launch_bounds__(512, 1)
 dense_cluster_kernel(const SysDev* __restrict__ sys, int nsys, int* queue, SmemPlan plan, SolveParams prm,
@@ -247,9 +247,9 @@ solve_kernel(const SysDev* __restrict__ sys, int nsys, int* queue, SmemPlan plan
 }
 
 // The merged slot array of one system, completed for callers that read the
-// factor in that layout: the engine's refactor stores the strict-L part
-// there (the later columns' gathers read it) and the U part, the diagonal
-// and the dense trailing block only in the arrays the solves read.  A CTA
+// factor in that layout: the engine's refactor stores the strict-L part there
+// and the U part, the diagonal and the dense trailing block only in the arrays
+// the solves read.  A CTA
 // per column (grid-stride).
 template <typename VT>
 __global__ void merge_factor_kernel(SysDev S) {
@@ -562,8 +562,7 @@ int refactor_block(const lusp_batch_opts& o, int nsys) {
     return nsys <= sm_count() ? 768 : 512;
 }
 
-void make_refactor_plan(const std::vector<PatternObj*>& pats, int threads, int vsize, SmemPlan& plan,
-                        int ctas_per_sm) {
+void make_refactor_plan(const std::vector<PatternObj*>& pats, int threads, SmemPlan& plan, int ctas_per_sm) {
     int nmax = 1, colmax = 2;
     for (auto* p : pats) {
         nmax = std::max(nmax, p->S.n);
@@ -584,7 +583,6 @@ void make_refactor_plan(const std::vector<PatternObj*>& pats, int threads, int v
     const size_t per_warp = budget > fixed ? (budget - fixed) / nw : 0;
     // Per warp: its column's record and pivot minima, and a work vector (wcap
     // fp64), the longest column when it fits.
-    (void)vsize;
     plan.wcap = (int)std::min<size_t>((size_t)colmax, per_warp > kWarpHead ? (per_warp - kWarpHead) / 8 : 0) & ~1;
     plan.bytes = fixed + (size_t)nw * (plan.wcap * 8 + kWarpHead);
 }
@@ -999,7 +997,7 @@ constexpr int kSpreadMidGroup = 12, kSpreadMidLeast = 6;
 
 int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& o, int nsys, LaunchArgs& a) {
     a.rblock = refactor_block(o, nsys);
-    make_refactor_plan(pats, a.rblock, o.prec == LUSP_FP64 ? 8 : 4, a.rplan);
+    make_refactor_plan(pats, a.rblock, a.rplan);
     int occ = 0;
     int rc = refactor_occupancy(o.prec, a.rplan.bytes, a.rblock, &occ);
     if (rc != LUSP_OK) return rc;
@@ -1045,7 +1043,7 @@ int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& 
             // 0.70 ms against one 2-CTA cluster each; the n = 989 circuit,
             // 41 k updates, gains nothing).
             SmemPlan pl;
-            make_refactor_plan(pats, 256, o.prec == LUSP_FP64 ? 8 : 4, pl);
+            make_refactor_plan(pats, 256, pl);
             int mocc = 0;
             rc = refactor_occupancy(o.prec, pl.bytes, 256, &mocc, true);
             if (rc != LUSP_OK) return rc;
@@ -1064,10 +1062,9 @@ int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& 
             int colsp = 2;
             for (auto* p : pats)
                 for (int k = 0; k < p->S.k0; k++) colsp = std::max(colsp, p->S.cp[k + 1] - p->S.cp[k]);
-            const int vs = o.prec == LUSP_FP64 ? 8 : 4;
             for (int t : {768, 512, 384, 256}) {
                 SmemPlan pl;
-                make_refactor_plan(pats, t, vs, pl, 1);
+                make_refactor_plan(pats, t, pl, 1);
                 if (pl.wcap >= colsp || t == 256) {
                     a.rblock = t;
                     a.rplan = pl;

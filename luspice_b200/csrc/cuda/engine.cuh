@@ -50,7 +50,7 @@ struct PatternDev {
     // Pattern of the dense trailing block, one bit per entry (row r, column c
     // of the block: bit c & 31 of word r * (tail_ld / 32) + c / 32).  The
     // refactor writes only these entries of the fp64 block; the dense kernel
-    // reads every other entry as 0 in its first panel step.
+    // reads every other entry as 0 when it loads a block column.
     const unsigned* tail_mask;
     // Column records of the refactorization, four 16-byte words per claim
     // index idx (column k = col_order[idx]): {k, cp[k], column length,

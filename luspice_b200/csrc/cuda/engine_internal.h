@@ -18,7 +18,7 @@ struct PatternObj {
     PatternDev desc{};               // host copy holding device pointers
     PatternDev* d_desc = nullptr;
     int* d_block = nullptr;
-    void* d_rel = nullptr;           // relative update slots (rel_ptr, rel)
+    void* d_rel = nullptr;           // relative update slots
     size_t bytes = 0;
 };
 
@@ -126,14 +126,13 @@ void fill_params(SolveParams& prm, const lusp_batch_opts& o);
 int plan_for(const std::vector<PatternObj*>& pats, const lusp_batch_opts& o, SmemPlan& plan);
 int kernel_occupancy(int prec, int inner, size_t smem, int block, int* occ);
 // spread: the spread-mode kernel (several CTAs per system, global-memory
-// synchronization) instead of the cluster kernel.
+// synchronization) instead of the one-CTA kernel.
 int refactor_occupancy(int prec, size_t smem, int block, int* occ, bool spread = false);
 int refactor_block(const lusp_batch_opts& o, int nsys);
 // Solve-kernel CTA size and plan target for nsys systems when left at 0.
 void resolve_solve_shape(lusp_batch_opts& o, int nsys);
 // ctas_per_sm: CTAs sharing an SM's shared memory (0: 1024 / threads).
-void make_refactor_plan(const std::vector<PatternObj*>& pats, int threads, int vsize, SmemPlan& plan,
-                        int ctas_per_sm = 0);
+void make_refactor_plan(const std::vector<PatternObj*>& pats, int threads, SmemPlan& plan, int ctas_per_sm = 0);
 // Refactorization kernel block, plan and grid for nsys systems of pats.
 int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& o, int nsys, LaunchArgs& a);
 // Kernels one launch with these RUN_* flags issues.

@@ -40,11 +40,6 @@ __device__ __forceinline__ int find_slot(const int* rows, int lo, int hi, int i)
     return (lo < end && rows[lo] == i) ? lo : -1;
 }
 
-// Non-blocking test of a ready bit.
-__device__ __forceinline__ bool is_ready(const unsigned* bits, int j) {
-    return (*((const volatile unsigned*)bits + (j >> 5)) >> (j & 31)) & 1u;
-}
-
 // Asynchronous global->shared copies (sm_80+ cp.async, L1-allocating):
 // issued without waiting, completed by cp_async_wait_all().
 __device__ __forceinline__ void cp_async_4(void* sdst, const void* gsrc) {
@@ -771,9 +766,8 @@ __device__ __forceinline__ void seg_update(const VT* lcol, const unsigned short*
 // into the system's sync area; the last CTA to finish writes the system's
 // statistics (pivot minima through the bit patterns of non-negative doubles:
 // a larger complement is a smaller value, so 0 means none yet).
-__device__ void spread_finish(const SysDev& S, unsigned* sync, int group, Smem& sm, double minpiv,
-                              double minratio, double maxu, int bad, long long cw, long long cg, long long cu,
-                              long long t_begin) {
+__device__ void spread_finish(const SysDev& S, unsigned* sync, int group, double minpiv, double minratio,
+                              double maxu, int bad, long long cw, long long cu, long long t_begin) {
     const int lane = threadIdx.x & 31;
     int* ctl = (int*)sync;
     unsigned long long* acc = (unsigned long long*)(sync + kSyncAcc);
@@ -787,12 +781,10 @@ __device__ void spread_finish(const SysDev& S, unsigned* sync, int group, Smem& 
         if (minratio < INFINITY) atomicMax(&acc[1], ~(unsigned long long)__double_as_longlong(minratio));
         atomicMax(&acc[2], (unsigned long long)__double_as_longlong(maxu));
         atomicAdd(&acc[3], (unsigned long long)cw);
-        atomicAdd(&acc[4], (unsigned long long)cg);
-        atomicAdd(&acc[5], (unsigned long long)cu);
+        atomicAdd(&acc[4], (unsigned long long)cu);
     }
     __threadfence();
     __syncthreads();
-    (void)sm;
     if (threadIdx.x == 0 && atomicAdd(&ctl[kSyncDone], 1) == group - 1) {
         __threadfence();
         const volatile unsigned long long* va = acc;
@@ -809,8 +801,8 @@ __device__ void spread_finish(const SysDev& S, unsigned* sync, int group, Smem& 
         st->inner_iters = 0;
         st->outer_iters = 0;
         st->cyc_wait = (long long)va[3];
-        st->cyc_gather = (long long)va[4];
-        st->cyc_update = (long long)va[5];
+        st->cyc_gather = 0;
+        st->cyc_update = (long long)va[4];
         st->cyc_refactor = clock64() - t_begin;
     }
 }
@@ -1165,7 +1157,7 @@ __device__ void refactor_phase(const RefactorCtx& cx, const SmemPlan& plan, char
     __syncwarp();
     const double minpiv = pmin[0], minratio = pmin[1];
     if (SPREAD) {
-        spread_finish(S, sync, group, sm, minpiv, minratio, maxu, bad, c_wait, 0, c_update, t_begin);
+        spread_finish(S, sync, group, minpiv, minratio, maxu, bad, c_wait, c_update, t_begin);
         return;
     }
     if (lane == 0) {
