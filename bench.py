@@ -715,9 +715,9 @@ def main():
     value = accepted * world / (step_ms / 1000.0)
     value64 = acc64 * world / (fp64_ms / 1000.0)
 
-    # Roofline of the dominant kernel: the sparse refactor kernel (the largest
-    # share of GPU time in the ncu launch list of this program), with the
-    # solve kernel beside it.  Each kernel's device time comes from CUDA
+    # Roofline of the dominant kernel: the solve kernel (the largest share of
+    # GPU time in the ncu launch list of this program), with the sparse
+    # refactor kernel beside it.  Each kernel's device time comes from CUDA
     # events the library records around it on the launching stream
     # (lusp_batch_time_kernels), L2 flushed before each timed launch.
     hbm, peak_kind = peaks()
@@ -741,6 +741,8 @@ def main():
         if sh["refactor_spread"] > 0:
             return (f"refactor_spread_kernel<float> ({sh['refactor_spread']} CTAs of {sh['refactor_block']} "
                     f"threads per system, {sh['refactor_grid']} CTAs)")
+        if sh["refactor_cluster"] <= 1:
+            return f"refactor_lone_kernel<float> (one CTA of {sh['refactor_block']} threads per system)"
         return (f"refactor_kernel<float> ({sh['refactor_cluster']}-CTA cluster of {sh['refactor_block']} threads "
                 f"per system, {sh['refactor_grid']} CTAs)")
 
@@ -881,15 +883,16 @@ def main():
                                         "pipelining": "copies of step k overlap kernels of step k-1 (two "
                                         "batches, two streams); kernels of consecutive steps serialized",
                                         "results_equal_device_timed": e2e_same}},
-            "roofline": {"bound": "hbm", "achieved": achieved_ref, "peak": hbm, "unit": "GB/s",
-                         "frac": achieved_ref / hbm,
-                         "traffic": traffic_of("refactor_spread_kernel_power_grid4050x50.json"),
-                         "peak_kind": peak_kind, "kernel": ref_kernel,
-                         "alg_bytes_per_launch": alg_ref, "kernel_ms": refactor_ms,
+            "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
+                         "frac": achieved / hbm,
+                         "traffic": traffic_of("solve_kernel_power_grid4050x50.json"),
+                         "peak_kind": peak_kind, "kernel": "solve_kernel<float, float>",
+                         "alg_bytes_per_launch": alg, "kernel_ms": solve_ms,
                          "dense_kernel_ms": dense_ms,
-                         "solve_kernel": {"achieved": achieved, "frac": achieved / hbm,
-                                          "traffic": traffic_of("solve_kernel_power_grid4050x50.json"),
-                                          "alg_bytes_per_launch": alg, "kernel_ms": solve_ms}},
+                         "refactor_kernel": {"kernel": ref_kernel, "achieved": achieved_ref,
+                                             "frac": achieved_ref / hbm,
+                                             "traffic": traffic_of("refactor_spread_kernel_power_grid4050x50.json"),
+                                             "alg_bytes_per_launch": alg_ref, "kernel_ms": refactor_ms}},
             "gpu_launches": launches,
             "clocks": clk.summary(),
             "cpu_baseline": cpu,

@@ -553,10 +553,14 @@ void resolve_solve_shape(lusp_batch_opts& o, int nsys) {
     if (o.ctas_per_sm <= 0) o.ctas_per_sm = few ? 1 : 2;
 }
 
-// One 768-thread CTA per SM (80 registers a thread, no spills in the
-// column loop) while every system has an SM or more; two 512-thread CTAs
-// per SM for wider batches (measured on B200: 768 is ~4% faster than 1024
-// threads on one SM, 512 x 2 ~24% faster than 256 x 4).
+// One 768-thread CTA per SM (80 registers a thread; 4-24 bytes spilled in
+// fp32, 140-148 in fp64) while every system has an SM or more; two 512-thread
+// CTAs per SM (64 registers; 144-172 and 260-328 bytes) for wider batches.
+// B200, us, one CTA per system with 512 / 768 / 1024 threads: 148 circuits
+// n = 3001 957 / 664 / 641, 148 grids n = 2000 1094 / 710 / 748; two CTAs of
+// 512 per SM against one of 768: 160 circuits n = 989 391 / 409, 320 656 / 613,
+// 640 1038 / 1040, 320 grids n = 2000 2401 / 2075 (256 threads: 638, 1253 and
+// 2434 for the last three).
 int refactor_block(const lusp_batch_opts& o, int nsys) {
     if (o.refactor_threads > 0) return o.refactor_threads;
     return nsys <= sm_count() ? 768 : 512;
@@ -978,9 +982,11 @@ void fill_params(SolveParams& prm, const lusp_batch_opts& o) {
 }
 
 // Gathered updates per system above which a batch of few systems spreads
-// each system's refactorization over many SMs (the n = 40,000 circuit has
-// 227 M; the n = 4050 power grid, refactored faster by one 2-SM cluster,
-// has 5.9 M).
+// each system's refactorization over all SMs, a CTA each (the n = 40,000
+// circuit has 227 M, the n = 4050 power grid 5.9 M).  B200, fp64, us, one
+// system over all SMs against 12 CTAs of 256 threads: n = 8000 with supply nets
+// (19 M) 2154 / 4853, n = 4000 (3.5 M, below the line, which was drawn for
+// slower updates) 861 / 1588.
 constexpr long long kSpreadMinUpdates = 16ll << 20;
 // Gathered updates per system above which a batch of at most one system
 // per SM spreads each system over up to kSpreadMidGroup 256-thread CTAs,
@@ -1004,8 +1010,10 @@ int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& 
     if (occ < 1) { set_error("refactor kernel does not fit one SM (smem %zu)", a.rplan.bytes); return LUSP_EARG; }
     a.rgrid = std::min(nsys, occ * sm_count());
     // Spread a system's columns over a cluster of CTAs when every system of
-    // the batch still gets its own cluster at once (the refactor is bound by
-    // instruction issue on one SM; the dependency chain leaves room).
+    // the batch still gets its own cluster at once.  B200, us, 50 systems on a
+    // cluster each / on one CTA each: n = 4050 grid 1311 / 1683, n = 3001
+    // circuit 511 / 630, n = 1500 294 / 328; the smallest pay for the distributed
+    // claims: n = 989 216 / 208, n = 400 127 / 92, n = 300 grid 96 / 68.
     a.rcluster = 1;
     int want = o.refactor_cluster;
     if (want == 0) want = (a.rblock > 512 && 2 * nsys <= sm_count()) ? 2 : 1;
@@ -1038,10 +1046,13 @@ int refactor_setup(const std::vector<PatternObj*>& pats, const lusp_batch_opts& 
         else if (nsys <= sm_count() && gmin >= kSpreadMidUpdates && o.refactor_threads <= 0 &&
                  o.refactor_cluster <= 0) {
             // Medium systems, at most one per SM: 256-thread CTAs, four per
-            // SM, up to kSpreadMidGroup per system (B200, 50 systems: the
-            // n = 4050 grid 2.22 -> 1.95 ms, an n = 4000 circuit 0.82 ->
-            // 0.70 ms against one 2-CTA cluster each; the n = 989 circuit,
-            // 41 k updates, gains nothing).
+            // SM, up to kSpreadMidGroup per system.  B200, us, 50 systems
+            // spread / on one 2-CTA cluster each / on one CTA each: n = 4050
+            // grid 971 / 1311 / 1683, n = 4000 circuit 484 / 684 / 858,
+            // n = 2000 circuit (149 k updates) 273 / 375 / 438, n = 500 grid
+            // (132 k) 106 / 128 / 104; below the line, with 8 CTAs each,
+            // n = 1500 circuit (118 k) 245 / 294 / 328, n = 989 (41 k)
+            // 184 / 216 / 208, n = 300 grid (48 k) 87 / 96 / 68.
             SmemPlan pl;
             make_refactor_plan(pats, 256, pl);
             int mocc = 0;

@@ -345,9 +345,10 @@ __device__ __noinline__ void dense_update_rows(double* xs, const double* xk, con
 // q - 4, so it is rolled and the current columns are registers 0..3.  Bound by
 // warp 0's chain (exchange, reciprocal 61, quotient 50, update 16 cycles a
 // column, and its own update's issue): 320 rows and 32 columns 24 k cycles
-// (B200); all warps in step, a barrier per column, 39 k; groups of four
-// pivots eliminated redundantly by every lane 34 k (two dependent divisions
-// per column instead of one).
+// (B200, alone; in the kernel a panel and its publication take 35 k on average
+// over a block of 320 and 48 k over one of 96); all warps in step, a barrier
+// per column, 39 k; groups of four pivots eliminated redundantly by every lane
+// 34 k (two dependent divisions per column instead of one).
 // ud: the pivot rows, entry (r, 4 (r / 4) + q) at ud + 34 r + q, the pivot's
 // reciprocal at ud + 34 r + 32.  vmax[c]: bits of the largest entry of column
 // c below the pivot before scaling, over the entries above the pivot in
